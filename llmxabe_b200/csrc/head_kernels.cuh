@@ -28,11 +28,11 @@ constexpr int kHeadMaxStages = 5;
 
 struct HeadLaunch {
     CUtensorMap tm_w;          // weight bytes [vocab][row_bytes / 4] as 32-bit words, box = box_w bytes x 64 rows
-    const __half* x_hi;        // [max_tokens][hidden]
-    const __half* x_lo;        // [max_tokens][hidden]
+    const float* x;            // [max_tokens][hidden]
     float* logits;             // [max_tokens][vocab]
     int* status;
     int vocab, hidden, tokens;
+    int x_vec;                 // x is 16-byte aligned
     int n_stages;
     uint32_t box_w, stage_bytes, x_stride;
 };
@@ -49,19 +49,6 @@ __host__ __device__ inline HeadSmem head_smem_layout(int n_stages, uint32_t stag
     R.bars = R.x_lo + 8u * x_stride;
     R.total = R.bars + 8u * 2u * kHeadMaxStages + 128u;  // + slack for aligning the base
     return R;
-}
-
-// x (fp32) -> hi = f16(x), lo = f16(x - hi).  grid: tokens.
-__global__ void k_head_split(const float* __restrict__ x, int tokens, int hidden, __half* __restrict__ hi,
-                             __half* __restrict__ lo) {
-    const int t = blockIdx.x;
-    if (t >= tokens) return;
-    for (int j = threadIdx.x; j < hidden; j += blockDim.x) {
-        const float v = x[(size_t)t * hidden + j];
-        const __half h = __float2half_rn(v);
-        hi[(size_t)t * hidden + j] = h;
-        lo[(size_t)t * hidden + j] = __float2half_rn(v - __half2float(h));
-    }
 }
 
 template <int QUANT>
@@ -91,24 +78,10 @@ __global__ void __launch_bounds__(32 * (1 + kStreamConsumerWarps), 1) k_head_row
         }
         fence_mbar_init();
     }
-    // this pass's activation rows (up to eight tokens), both parts; rows past the batch are zero
-    const int t0 = (int)blockIdx.y * 8;
-    const int ncols = min(8, P.tokens - t0);
-    {
-        const int words_per_row = P.hidden / 2;  // two f16 per word
-        for (int i = threadIdx.x; i < 8 * words_per_row; i += blockDim.x) {
-            const int c = i / words_per_row, j = i - c * words_per_row;
-            uint32_t vh = 0u, vl = 0u;
-            if (c < ncols) {
-                vh = ((const uint32_t*)(P.x_hi + (size_t)(t0 + c) * P.hidden))[j];
-                vl = ((const uint32_t*)(P.x_lo + (size_t)(t0 + c) * P.hidden))[j];
-            }
-            *(uint32_t*)(smem + lay.x_hi + (uint32_t)c * P.x_stride + 4u * j) = vh;
-            *(uint32_t*)(smem + lay.x_lo + (uint32_t)c * P.x_stride + 4u * j) = vl;
-        }
-    }
     __syncthreads();
     volatile int* abortp = &abort_flag;
+    const int t0 = (int)blockIdx.y * 8;
+    const int ncols = min(8, P.tokens - t0);
     const int n_spans = P.hidden / kSpanElems;
     const int units = (P.vocab + kHeadUnitRows - 1) / kHeadUnitRows;
     const int span_b = span_bytes_of(QUANT);
@@ -142,6 +115,35 @@ __global__ void __launch_bounds__(32 * (1 + kStreamConsumerWarps), 1) k_head_row
     }
 
     // ---------------------------------- consumers ----------------------------------
+    // This pass's activation rows (up to eight tokens) as hi = f16(x) and lo = f16(x - hi); rows past the
+    // batch are zero.  The weight ring fills meanwhile.  (A launch of its own that wrote both parts to
+    // memory first cost 5 us plus its launch; each CTA reads the same number of bytes either way.)
+    {
+        const int quads = P.hidden / 4;
+        for (int i = threadIdx.x - 32; i < 8 * quads; i += 32 * kStreamConsumerWarps) {
+            const int c = i / quads, j = i - c * quads;
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            if (c < ncols) {
+                const float* src = P.x + (size_t)(t0 + c) * P.hidden + 4 * j;
+                if (P.x_vec) {
+                    const float4 q = *(const float4*)src;
+                    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) v[k] = src[k];
+                }
+            }
+            __half2 h[2], l[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                h[k] = __floats2half2_rn(v[2 * k], v[2 * k + 1]);
+                l[k] = __floats2half2_rn(v[2 * k] - __low2float(h[k]), v[2 * k + 1] - __high2float(h[k]));
+            }
+            *(uint2*)(smem + lay.x_hi + (uint32_t)c * P.x_stride + 8u * j) = *(const uint2*)h;
+            *(uint2*)(smem + lay.x_lo + (uint32_t)c * P.x_stride + 8u * j) = *(const uint2*)l;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kStreamConsumerWarps) : "memory");  // the consumer warps only
+    }
     const int cw = warp - 1;
     const int gi = cw / kStreamGroupWarps;
     const int w = cw % kStreamGroupWarps;
@@ -188,50 +190,78 @@ __global__ void __launch_bounds__(32 * (1 + kStreamConsumerWarps), 1) k_head_row
 }
 
 // Index of the largest of n values, ties to the lower index (gemv.rs:102-111; the reference's
-// device form is LmHeadKernels::argmax, lm_head.rs:1950-2015).  One block per row of `logits`.
-__global__ void __launch_bounds__(1024) k_head_argmax(const float* __restrict__ logits, int vocab, int tokens,
-                                                      int* __restrict__ out) {
-    __shared__ float bv[32];
-    __shared__ int bi[32];
-    const int tk = blockIdx.x;
-    if (tk >= tokens) return;
+// device form is LmHeadKernels::argmax, lm_head.rs:1950-2015).  A row of `logits` is shared out over a
+// cluster of eight CTAs, whose candidates meet in the first CTA's shared memory, so no scratch outlives
+// the launch.  One CTA per row with one load in flight per thread took 100 us for 3 rows of 248,320
+// (1 MB through one SM at 10 GB/s); eight CTAs with eight loads in flight each take 5 us.
+// grid: tokens x kArgmaxSplits, block kArgmaxThreads.
+constexpr int kArgmaxSplits = 8;  // the portable cluster size
+constexpr int kArgmaxThreads = 512;
+
+// (best, idx) <- the better of it and (ob, oi).  Comparisons with a NaN are false: a NaN never replaces
+// anything, and a NaN in front (index 0) is never replaced, as in the reference's scan.
+__device__ __forceinline__ void argmax_take(float& best, int& idx, float ob, int oi) {
+    if (ob > best || (ob == best && oi < idx)) {
+        best = ob;
+        idx = oi;
+    }
+}
+__device__ __forceinline__ void argmax_warp(float& best, int& idx) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+        argmax_take(best, idx, __shfl_xor_sync(0xffffffffu, best, off), __shfl_xor_sync(0xffffffffu, idx, off));
+}
+
+__global__ void __cluster_dims__(kArgmaxSplits, 1, 1) __launch_bounds__(kArgmaxThreads)
+    k_head_argmax(const float* __restrict__ logits, int vocab, int tokens, int* __restrict__ out) {
+    __shared__ float bv[32], cv[kArgmaxSplits];
+    __shared__ int bi[32], ci[kArgmaxSplits];
+    const int tk = blockIdx.x / kArgmaxSplits, part = blockIdx.x % kArgmaxSplits;  // part: the CTA's rank in its cluster
     const float* v = logits + (size_t)tk * vocab;
+    const int per = (vocab + kArgmaxSplits - 1) / kArgmaxSplits;
+    const int lo = part * per, hi = min(vocab, lo + per);
+    // every thread starts from element 0, which is a valid candidate
     float best = v[0];
     int idx = 0;
-    for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
-        const float x = v[i];
-        if (x > best || (x == best && i < idx)) {
-            best = x;
-            idx = i;
+    constexpr int U = 8;
+    for (int i0 = lo + threadIdx.x; i0 < hi; i0 += U * kArgmaxThreads) {
+        float x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * kArgmaxThreads;
+            x[u] = i < hi ? v[i] : 0.f;
         }
-    }
-    // a thread that saw nothing larger than v[0] holds (v[0], 0), which is a valid candidate
-    for (int off = 16; off > 0; off >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-        if (ob > best || (ob == best && oi < idx)) {
-            best = ob;
-            idx = oi;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * kArgmaxThreads;
+            if (i < hi) argmax_take(best, idx, x[u], i);
         }
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    argmax_warp(best, idx);
     if (lane == 0) {
         bv[warp] = best;
         bi[warp] = idx;
     }
     __syncthreads();
     if (warp == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        best = lane < nw ? bv[lane] : bv[0];
-        idx = lane < nw ? bi[lane] : bi[0];
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-            if (ob > best || (ob == best && oi < idx)) {
-                best = ob;
-                idx = oi;
-            }
+        constexpr int NW = kArgmaxThreads / 32;
+        best = bv[lane % NW];
+        idx = bi[lane % NW];
+        argmax_warp(best, idx);
+        if (lane == 0) {  // into slot `part` of the cluster's first CTA
+            uint32_t a, b;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(&cv[part])));
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(b) : "r"(smem_u32(&ci[part])));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(best) : "memory");
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(b), "r"(idx) : "memory");
         }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (part == 0 && warp == 0) {
+        best = cv[lane % kArgmaxSplits];
+        idx = ci[lane % kArgmaxSplits];
+        argmax_warp(best, idx);
         if (lane == 0) out[tk] = idx;
     }
 }

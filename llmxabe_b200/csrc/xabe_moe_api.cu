@@ -2092,8 +2092,6 @@ struct xabe_lm_head {
     xabe_lm_head_geometry g{};
     int device = 0;
     int sm_count = 0;
-    __half* x_hi = nullptr;  // [max_tokens][hidden]
-    __half* x_lo = nullptr;
     int* status = nullptr;   // device word the bounded waits write
     int* h_status = nullptr; // pinned
 };
@@ -2128,10 +2126,7 @@ int xabe_lm_head_create(const xabe_lm_head_geometry* geometry, int device, xabe_
     m->g = g;
     m->device = device;
     m->sm_count = prop.multiProcessorCount;
-    const size_t n = (size_t)g.max_tokens * g.hidden;
-    cudaError_t e = cudaMalloc(&m->x_hi, n * sizeof(__half));
-    if (e == cudaSuccess) e = cudaMalloc(&m->x_lo, n * sizeof(__half));
-    if (e == cudaSuccess) e = cudaMalloc(&m->status, sizeof(int));
+    cudaError_t e = cudaMalloc(&m->status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(m->status, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&m->h_status, sizeof(int));
     if (e != cudaSuccess) {
@@ -2145,8 +2140,6 @@ int xabe_lm_head_create(const xabe_lm_head_geometry* geometry, int device, xabe_
 void xabe_lm_head_destroy(xabe_lm_head* m) {
     if (!m) return;
     cudaSetDevice(m->device);
-    cudaFree(m->x_hi);
-    cudaFree(m->x_lo);
     cudaFree(m->status);
     if (m->h_status) cudaFreeHost(m->h_status);
     delete m;
@@ -2185,8 +2178,8 @@ int xabe_lm_head_forward(xabe_lm_head* m, void* stream, xabe_quant_tensor weight
     P.box_w = rows_box_bytes(q);
     int rc = make_bytes_map(&P.tm_w, weight.dev_bytes, g.vocab, row_bytes, P.box_w);
     if (rc) return rc;
-    P.x_hi = m->x_hi;
-    P.x_lo = m->x_lo;
+    P.x = hidden_states;
+    P.x_vec = ((uintptr_t)hidden_states & 15) == 0;
     P.logits = logits;
     P.status = m->status;
     P.vocab = (int)g.vocab;
@@ -2204,8 +2197,6 @@ int xabe_lm_head_forward(xabe_lm_head* m, void* stream, xabe_quant_tensor weight
     }
     if (!smem) return fail(XABE_ERR_UNSUPPORTED_GEOMETRY, "LM head pass does not fit shared memory");
     cudaStream_t st = (cudaStream_t)stream;
-    k_head_split<<<tokens, 256, 0, counted(st)>>>(hidden_states, tokens, (int)g.hidden, m->x_hi, m->x_lo);
-    CUDA_TRY(cudaGetLastError());
     const dim3 grid(m->sm_count, (tokens + 7) / 8), block(32 * (1 + kStreamConsumerWarps));
     if (q == QUANT_Q6K) {
         CUDA_TRY(allow_dynamic_smem((const void*)k_head_rows<QUANT_Q6K>, smem));
@@ -2228,7 +2219,7 @@ int xabe_lm_head_argmax(xabe_lm_head* m, void* stream, const float* logits, size
         return fail(XABE_ERR_BUFFER_LENGTH, "logits must hold %zu floats, holds %zu",
                     (size_t)m->g.max_tokens * m->g.vocab, logits_len);
     if (tokens == 0) return XABE_OK;
-    k_head_argmax<<<tokens, 1024, 0, counted((cudaStream_t)stream)>>>(logits, (int)m->g.vocab, tokens, out);
+    k_head_argmax<<<tokens * kArgmaxSplits, kArgmaxThreads, 0, counted((cudaStream_t)stream)>>>(logits, (int)m->g.vocab, tokens, out);
     CUDA_TRY(cudaGetLastError());
     return XABE_OK;
 }
