@@ -340,18 +340,32 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
 }
 
 // out[t][j] = sum over ascending ks of partial[ks][t][j] for the live rows (MODE_DOWN with several
-// shares of the contraction).  grid: (max_tokens, ceil(rows / 256)), block 256.
+// shares of the contraction), and, when `residual` is given, the block's last stage
+// l_out = out + residual.  The shares' loads are all in flight before the first sum.
+// grid: (max_tokens, ceil(rows / 256)), block 256.
 __global__ void __launch_bounds__(256) k_sum_k_splits(const float* __restrict__ partial, int k_splits,
                                                       int max_tokens, int rows,
                                                       const int* __restrict__ valid_tokens,
-                                                      float* __restrict__ out) {
+                                                      float* __restrict__ out, const float* __restrict__ residual,
+                                                      float* __restrict__ l_out) {
     const int tk = blockIdx.x;
     if (tk >= *valid_tokens) return;
     const int j = blockIdx.y * 256 + threadIdx.x;
     if (j >= rows) return;
+    const size_t o = (size_t)tk * rows + j;
+    const float res = residual ? residual[o] : 0.0f;
     float r = 0.0f;
-    for (int ks = 0; ks < k_splits; ++ks) r += partial[((size_t)ks * max_tokens + tk) * rows + j];
-    out[(size_t)tk * rows + j] = r;
+    for (int k0 = 0; k0 < k_splits; k0 += 8) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < k_splits) v[k] = partial[(size_t)(k0 + k) * max_tokens * rows + o];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < k_splits) r += v[k];
+    }
+    out[o] = r;
+    if (residual) l_out[o] = r + res;
 }
 
 }  // namespace xabe

@@ -59,11 +59,13 @@ __global__ void k_rms_norm(const float* __restrict__ x, const float* __restrict_
     }
 }
 
-// k_rms_norm for many rows: the same sums in the same order, but a block walks rows blockIdx.x,
-// + gridDim.x, ... with the NEXT row's elements already on their way while it reduces the current one,
-// and keeps a row's elements in registers between the sum and the scaling (one read of x instead of
-// two).  One block per row spends most of a row's time waiting for its first load: 16384 rows of 2048
-// took 160 us where the 335 MB they move need 52 us.
+// k_rms_norm without the gate, for rows of at most eight elements per thread: the same sums in the same
+// order, but a block walks rows blockIdx.x, + gridDim.x, ... with the NEXT row's elements already on
+// their way while it reduces the current one, and keeps a row's elements in registers between the sum
+// and the scaling (one read of x instead of two).  One block per row spends most of a row's time waiting
+// for its first load: 16384 rows of 2048 took 160 us where the 335 MB they move need 52 us.  At decode
+// widths (a block has one row) what counts is that the row and the weights arrive together, before the
+// sum, instead of in two dependent passes of load loops: one row of 5120 took 7 us.
 // EPT: elements per thread = ceil(width / blockDim.x), at most 8.  grid: a few blocks per SM.
 template <int EPT>
 __global__ void __launch_bounds__(1024) k_rms_norm_stream(const float* __restrict__ x, const float* __restrict__ weight,
@@ -1303,13 +1305,29 @@ __global__ void __launch_bounds__(256) k_ep_combine(
 }
 
 // Dense FFN epilogue (crates/xabe-engine/src/block/dense_ffn.rs:234-251):
-// l_out = ffn_out + residual for the live rows.
-__global__ void k_add_residual(const float* __restrict__ ffn, const float* __restrict__ residual,
-                               const int* __restrict__ valid_tokens, int hidden, float* __restrict__ l_out) {
-    int t = blockIdx.x;
+// l_out = ffn_out + residual for the live rows.  HBM-bound at prefill widths; at one token only latency
+// counts, so a row is shared out over blocks with four loads in flight per thread (one block per row that
+// walked it element by element took 11 us at any decode width).
+// grid: (max_tokens, ceil(hidden / 1024)), block 256.
+__global__ void __launch_bounds__(256) k_add_residual(const float* __restrict__ ffn, const float* __restrict__ residual,
+                                                      const int* __restrict__ valid_tokens, int hidden,
+                                                      float* __restrict__ l_out) {
+    const int t = blockIdx.x;
     if (t >= *valid_tokens) return;
-    size_t base = (size_t)t * hidden;
-    for (int j = threadIdx.x; j < hidden; j += blockDim.x) l_out[base + j] = ffn[base + j] + residual[base + j];
+    const size_t base = (size_t)t * hidden;
+    const int j0 = blockIdx.y * 1024 + threadIdx.x;
+    float f[4], r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int j = j0 + 256 * i;
+        f[i] = j < hidden ? ffn[base + j] : 0.f;
+        r[i] = j < hidden ? residual[base + j] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int j = j0 + 256 * i;
+        if (j < hidden) l_out[base + j] = f[i] + r[i];
+    }
 }
 
 // bf16 rows -> fp32 rows for the live tokens: the widening is a 16-bit shift,

@@ -517,6 +517,14 @@ struct TailFusion {
     float* l_out;
 };
 
+// The dense block's last stage (l_out = ffn_out + residual): `done` says that the launches of the
+// projections performed it already.
+struct DenseTail {
+    const float* residual;
+    float* l_out;
+    bool done = false;
+};
+
 bool tail_applies(const xabe_moe* m, const xabe_moe_layer_weights* w) {
     const auto& g = m->g;
     // Handles of fewer than 16 tokens: the routed and the shared experts always share one launch there
@@ -531,7 +539,7 @@ bool tail_applies(const xabe_moe* m, const xabe_moe_layer_weights* w) {
 // Both projections of the routed experts and/or the shared expert, each in one
 // launch.  `routed`/`shared` say which halves ride the launch.
 int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const MlpWeights& shared,
-                float* shexp_out, int mark_between = -1, const TailFusion* tail = nullptr) {
+                float* shexp_out, int mark_between = -1, const TailFusion* tail = nullptr, DenseTail* dense = nullptr) {
     const auto& g = m->g;
     if (!routed.present && !shared.present) return XABE_OK;
     // Different formats for the routed experts and the shared expert (the shipped file: Q6_K and Q8_0):
@@ -631,8 +639,10 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
             if ((rc = launch_dense_rows<MODE_DOWN>(m, st, P, qd, ng, smem))) return rc;
             if (P.k_splits > 1) {
                 k_sum_k_splits<<<dim3(g.max_tokens, (g.hidden + 255) / 256), 256, 0, counted(st)>>>(
-                    m->dense_partial, P.k_splits, (int)g.max_tokens, (int)g.hidden, m->valid_tokens, shexp_out);
+                    m->dense_partial, P.k_splits, (int)g.max_tokens, (int)g.hidden, m->valid_tokens, shexp_out,
+                    dense ? dense->residual : nullptr, dense ? dense->l_out : nullptr);
                 CUDA_TRY(cudaGetLastError());
+                if (dense) dense->done = true;
             }
             return XABE_OK;
         }
@@ -861,9 +871,8 @@ int launch_rms_norm(xabe_moe* m, cudaStream_t st, const float* x, const float* w
     if (block < 32) block = 32;
     if (gate_w && block < 256) gate_w = nullptr;  // (hidden is a multiple of 256, so this does not happen)
     const size_t smem = gate_w ? (size_t)m->g.hidden * sizeof(float) : 0;
-    // many rows: blocks that walk rows with the next row's loads in flight (same sums, same order)
     const int ept = ((int)m->g.hidden + block - 1) / block;
-    if (!gate_w && m->g.max_tokens >= 256 && ept <= 8) {
+    if (!gate_w && ept <= 8) {
         const dim3 grid((unsigned)std::min<uint32_t>(m->g.max_tokens, 2u * (uint32_t)m->sm_count));
         auto go = [&](auto kern) -> int {
             CUDA_TRY(launch_pdl(m->pdl, kern, grid, dim3(block), 0, st, x, weight, m->normed, m->normed_h,
@@ -1780,8 +1789,11 @@ int xabe_dense_ffn_block_forward(xabe_moe* m, void* stream, const float* post_no
     s.gate = gate;
     s.up = up;
     s.down = down;
-    if ((rc = run_experts(m, st, MlpWeights{}, s, ffn_out))) return rc;
-    k_add_residual<<<g.max_tokens, 256, 0, counted(st)>>>(ffn_out, residual, m->valid_tokens, (int)g.hidden, l_out);
+    DenseTail tail{residual, l_out};
+    if ((rc = run_experts(m, st, MlpWeights{}, s, ffn_out, -1, nullptr, &tail))) return rc;
+    if (tail.done) return XABE_OK;
+    k_add_residual<<<dim3(g.max_tokens, (g.hidden + 1023) / 1024), 256, 0, counted(st)>>>(
+        ffn_out, residual, m->valid_tokens, (int)g.hidden, l_out);
     CUDA_TRY(cudaGetLastError());
     return XABE_OK;
 }
