@@ -303,7 +303,7 @@ int xabe_moe_force_prefill_path(xabe_moe* m, int on);
 
 /* Per-handle tuning switches; none changes a result, only which launch shape produces it.  They
  * replace process-wide environment reads: a host with several handles sets each one's own.
- * PREFILL_WIDE allocates (set-up time only); the others are plain field writes. */
+ * All are plain field writes. */
 #define XABE_TUNE_PDL 0                /* 1: programmatic dependent launch between the block's kernels */
 #define XABE_TUNE_STREAM_STAGES 1      /* ring depth cap of the streaming kernels (0 = as many as fit) */
 #define XABE_TUNE_STREAM_RUNS 2        /* k_expert_stream work split override (0 = the kernel's choice) */
@@ -311,8 +311,7 @@ int xabe_moe_force_prefill_path(xabe_moe* m, int on);
 #define XABE_TUNE_ROUTER_REGW 4        /* router kernel with expert rows in registers: 0 off, 1 sixteen rows per CTA
                                           (one CTA per SM), 2 eight rows (two CTAs per SM), -1 by width (from 256 tokens: 2) */
 #define XABE_TUNE_FORCE_TILE_KERNELS 5 /* 1: the one-tile-per-CTA expert kernels everywhere */
-#define XABE_TUNE_PREFILL_WIDE 6       /* 1 or 4: k_prefill_gemm_wide with up to four 128-column accumulators per unpacked
-                                          weight pair; 2, 3: up to two or three; 0: k_prefill_gemm (one) */
+#define XABE_TUNE_PREFILL_WIDE 6       /* accepted, without effect: one prefill kernel serves every width */
 #define XABE_TUNE_FUSED_DECODE 7       /* bit 0: handles under 16 tokens fold gate-and-combine into the down launch;
                                           bit 1: handles up to 256 tokens run norm, router, routing and dispatch as one
                                           launch.  3 = a three-launch layer at up to 15 tokens; both measured no

@@ -9,6 +9,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <new>
+#include <algorithm>
 #include <string>
 #include <utility>
 
@@ -20,7 +21,7 @@
 #include "stream_rows_kernels.cuh"
 #include "head_kernels.cuh"
 #include "ep_kernels.cuh"
-#include "prefill_wide_kernels.cuh"
+#include "prefill_kernels.cuh"
 #include "dense_rows_kernels.cuh"
 
 using namespace xabe;
@@ -92,9 +93,6 @@ cudaError_t launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, 
     cfg.numAttrs = off ? 0 : 1;
     return cudaLaunchKernelEx(&cfg, kern, KArgs(std::forward<Args>(args))...);
 }
-
-// Handles sized for this many tokens use k_prefill_gemm_wide (set from measurements).
-constexpr uint32_t kPrefillWideMinTokens = 1024;
 
 // Wide passes only take the tcgen05 prefill kernels; the launch shape comes from max_tokens.
 constexpr uint32_t kPrefillMinTokens = 512;
@@ -168,7 +166,6 @@ struct xabe_moe {
     int* pf_items = nullptr;    // token tiles for the tcgen05 prefill kernels
     int* pf_n_items = nullptr;
     uint64_t pf_capacity = 0;
-    int pf_item_cols = 128;     // token columns per item: 128 (k_prefill_gemm) or 512 (k_prefill_gemm_wide)
     // per-handle switches (xabe_moe_set_tuning, xabe_moe_disable_tensor_cores, xabe_moe_force_prefill_path)
     bool force_tile_kernels = false;  // use the one-tile-per-CTA kernels even where the streaming ones apply
     bool pdl = false;                 // programmatic dependent launch between the block's kernels
@@ -196,8 +193,6 @@ struct xabe_moe {
     int* ep_compact = nullptr;  // [num_experts + 1] live pairs before each expert (expert parallelism)
     int* ep_rank_start = nullptr;   // [kEpMaxRanks] where each rank's pairs start in the send order
     int* ep_send_counts = nullptr;  // [kEpMaxRanks]
-    __half* x_sorted = nullptr;  // activations in dispatch order (k_prefill_gemm_wide's routed gate/up source)
-    CUtensorMap tm_routed_gu{}, tm_routed_dn{}, tm_shared_gu{}, tm_shared_dn{};
     float* const* partial_rows = nullptr;  // optional per-row destinations of the down projection (expert parallelism)
     const __half* x_routed_override = nullptr;  // caller-provided f16 rows for one grouped pass
     float* logits = nullptr;
@@ -363,34 +358,18 @@ EncodeTiledFn encode_tiled_fn() {
     }
     return fn;
 }
-// [rows][k] f16 row-major, box 64 elements x 128 rows, 128-byte swizzle, out-of-bounds rows read as zero.
-int make_rows_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t k) {
-    EncodeTiledFn enc = encode_tiled_fn();
-    if (!enc) return fail(XABE_ERR_DRIVER, "cuTensorMapEncodeTiled is not available from this driver");
-    if (((uintptr_t)base & 15) != 0 || k % 64 != 0 || rows == 0)
-        return fail(XABE_ERR_INVALID_ARGUMENT, "tensor map source must be 16-byte aligned with k a multiple of 64");
-    cuuint64_t dims[2] = {k, rows};
-    cuuint64_t strides[1] = {k * 2};
-    cuuint32_t box[2] = {(cuuint32_t)kPfChunkK, (cuuint32_t)kPfTileN};
-    cuuint32_t elem[2] = {1, 1};
-    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(XABE_ERR_DRIVER, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    return XABE_OK;
-}
-
 // Weight bytes as a matrix [rows][row_bytes / 4] of 32-bit words (a box side is limited to 256
-// elements, and a Q8_0 span is 272 bytes), box `box_w` bytes x 64 rows, no swizzle; the part of a
+// elements, and a Q8_0 span is 272 bytes), box `box_w` bytes x `box_rows` rows, no swizzle; the part of a
 // box past the end of a row reads as zero.
-int make_bytes_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_w) {
+int make_bytes_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_w,
+                   uint32_t box_rows = kRowsGroupRows) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return fail(XABE_ERR_DRIVER, "cuTensorMapEncodeTiled is not available from this driver");
     if (((uintptr_t)base & 15) != 0 || row_bytes % 16 != 0 || rows == 0 || box_w % 16 != 0 || box_w > 1024)
         return fail(XABE_ERR_INVALID_ARGUMENT, "weight tensor map needs a 16-byte aligned base and row pitch");
     cuuint64_t dims[2] = {row_bytes / 4, rows};
     cuuint64_t strides[1] = {row_bytes};
-    cuuint32_t box[2] = {box_w / 4, (cuuint32_t)kRowsGroupRows};
+    cuuint32_t box[2] = {box_w / 4, box_rows};
     cuuint32_t elem[2] = {1, 1};
     CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, elem,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -451,7 +430,7 @@ int launch_rows_t(xabe_moe* m, cudaStream_t st, const RowsLaunch& P, uint32_t sm
 
 bool prefill_applies(const xabe_moe* m, int gateup_rows, int down_rows, int hidden, int inter) {
     if (m->force_tile_kernels || !m->tensor_cores) return false;
-    if (!(gateup_rows % 64 == 0 && down_rows % kPfTileM == 0 && hidden % kSpanElems == 0 && inter % kSpanElems == 0))
+    if (!(gateup_rows % kPfTileM == 0 && down_rows % (2 * kPfTileM) == 0 && hidden % kSpanElems == 0 && inter % kSpanElems == 0))
         return false;
     // Contractions too long for the decode kernels (the dense 27B block: 5120 and 17408) go through
     // these kernels at every width; there the exact-decode switch has nothing to select.
@@ -463,21 +442,38 @@ bool prefill_applies(const xabe_moe* m, int gateup_rows, int down_rows, int hidd
     return m->g.max_tokens >= kPrefillMinTokens;
 }
 
+// The tensor map k_prefill_gemm reads a weight stack of `rows` rows of `k` elements through.
+int make_prefill_map(CUtensorMap* out, const void* base, uint64_t rows, int k, int quant) {
+    const int q = quant == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0;
+    const uint32_t row_bytes = (uint32_t)(k / kSpanElems * span_bytes_of(q));
+    const int R = pf_row_group(row_bytes);
+    return make_bytes_map(out, base, rows / R, (uint64_t)row_bytes * R, rows_box_bytes(q),
+                          (uint32_t)std::min(32, kPfTileM / R));
+}
+
 template <int MODE, int QR, int QS>
-int launch_prefill_t(cudaStream_t st, const PrefillLaunch& L, dim3 grid, size_t smem, bool wide) {
-    auto kern = wide ? k_prefill_gemm_wide<MODE, QR, QS> : k_prefill_gemm<MODE, QR, QS>;
+int launch_prefill_t(xabe_moe* m, cudaStream_t st, const PrefillLaunch& L, uint32_t smem) {
+    auto kern = k_prefill_gemm<MODE, QR, QS>;
     CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-    kern<<<grid, wide ? kPfWideThreads : kPfThreads, smem, counted(st)>>>(L);
+    kern<<<m->sm_count, kPfThreads, smem, counted(st)>>>(L);
     CUDA_TRY(cudaGetLastError());
     return XABE_OK;
 }
 template <int MODE>
-int launch_prefill(cudaStream_t st, const PrefillLaunch& L, dim3 grid, size_t smem, int qr, int qs, bool wide) {
+int launch_prefill(xabe_moe* m, cudaStream_t st, PrefillLaunch& L, int qr, int qs) {
+    // one CTA per SM; the B ring takes what the raw slots of the longer row format leave
+    int box = 0;
+    if (L.has_routed) box = (int)rows_box_bytes(qr == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
+    if (L.has_shared) box = std::max(box, (int)rows_box_bytes(qs == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0));
+    L.slot_bytes = 32 * box;
+    L.n_b = kPfMaxBStages;
+    while (L.n_b > 2 && pf_smem_bytes(L.slot_bytes, L.n_b) > 223u * 1024u) --L.n_b;
+    const uint32_t smem = pf_smem_bytes(L.slot_bytes, L.n_b);
     if (qr == XABE_QUANT_Q6_K)
-        return qs == XABE_QUANT_Q6_K ? launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q6K>(st, L, grid, smem, wide)
-                                     : launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q8_0>(st, L, grid, smem, wide);
-    return qs == XABE_QUANT_Q6_K ? launch_prefill_t<MODE, QUANT_Q8_0, QUANT_Q6K>(st, L, grid, smem, wide)
-                                 : launch_prefill_t<MODE, QUANT_Q8_0, QUANT_Q8_0>(st, L, grid, smem, wide);
+        return qs == XABE_QUANT_Q6_K ? launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q6K>(m, st, L, smem)
+                                     : launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q8_0>(m, st, L, smem);
+    return qs == XABE_QUANT_Q6_K ? launch_prefill_t<MODE, QUANT_Q8_0, QUANT_Q6K>(m, st, L, smem)
+                                 : launch_prefill_t<MODE, QUANT_Q8_0, QUANT_Q8_0>(m, st, L, smem);
 }
 
 // ---- decode-width dense block (k_dense_rows) -------------------------------------------
@@ -663,61 +659,36 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
         P.partial_rows = m->partial_rows;
         P.shexp = shexp_out;
         P.status = m->status;
-        P.max_tokens = (int)g.max_tokens;
-        P.n_stages = kPfMaxStages;
-        P.item_cols = m->pf_item_cols;
-        const bool wide = m->pf_item_cols > kPfTileN;
-        // one CTA per SM walks the tiles; the rings take what fits beside each other
-        dim3 pf_grid((unsigned)m->sm_count);
-        auto pf_smem = [&](int q_routed, int q_shared) {
-            int pitch = 0;
-            if (routed.present) pitch = pf_raw_pitch(q_routed == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
-            if (shared.present) {
-                int ps = pf_raw_pitch(q_shared == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
-                if (ps > pitch) pitch = ps;
-            }
-            P.slot_bytes = kPfTileM * pitch;
-            if (wide) {  // A ring 64 KB, two raw slots, B ring three units (two beside the longer Q8_0 rows)
-                P.n_raw = kPfWideRaw;
-                P.n_b_units = pitch == kPfRawPitchQ6K ? kPfWideMaxBUnits : 2;
-                return (size_t)1024 + (size_t)(2 + P.n_b_units) * 2 * kPfTileBytes + (size_t)P.n_raw * P.slot_bytes + 16;
-            }
-            P.n_raw = pitch == kPfRawPitchQ6K ? kPfMaxRaw : 2;
-            return (size_t)1024 + (size_t)P.n_stages * kPfStageBytes + (size_t)P.n_raw * P.slot_bytes + 16;
-        };
-        P.r_a = L.r_a; P.r_b = L.r_b; P.s_a = L.s_a; P.s_b = L.s_b;
         P.rows = (int)g.intermediate; P.k = (int)g.hidden;
         P.x_routed = x_routed; P.x_shared = m->normed_h;
-        P.row_tiles = (int)g.intermediate / 64;
-        const size_t smem_gu = pf_smem(qr, qs);
-        if (wide) {
-            P.tm_routed = m->tm_routed_gu;
-            P.tm_shared = m->tm_shared_gu;
-            if (routed.present) {  // activation rows in dispatch order, so that an item's columns are consecutive rows
-                k_permute_rows<<<(unsigned)m->sorted_capacity, 256, 0, counted(st)>>>(
-                    m->sorted_token_ids, m->num_tokens_post_pad, m->valid_tokens, (int)g.experts_per_token,
-                    (int)g.hidden, x_routed, m->x_sorted);
-                CUDA_TRY(cudaGetLastError());
-            }
+        P.row_units = (int)g.intermediate / kPfTileM;
+        const uint64_t E = g.num_experts;
+        int rcp = XABE_OK;
+        if (routed.present) {
+            rcp = make_prefill_map(&P.tm_r_a, L.r_a, E * g.intermediate, P.k, qr);
+            if (!rcp) rcp = make_prefill_map(&P.tm_r_b, L.r_b, E * g.intermediate, P.k, qr);
         }
-        int rcp = launch_prefill<MODE_GATEUP>(st, P, pf_grid, smem_gu, qr, qs, wide);
+        if (!rcp && shared.present) {
+            rcp = make_prefill_map(&P.tm_s_a, L.s_a, g.intermediate, P.k, qs);
+            if (!rcp) rcp = make_prefill_map(&P.tm_s_b, L.s_b, g.intermediate, P.k, qs);
+        }
+        if (!rcp) rcp = launch_prefill<MODE_GATEUP>(m, st, P, qr, qs);
         if (rcp) return rcp;
         if (mark_between >= 0) prof_mark(m, st, mark_between);
-        int qrd = routed.present ? routed.down.quant : shared.down.quant;
-        int qsd = shared.present ? shared.down.quant : qrd;
-        P.r_a = routed.present ? (const uint8_t*)routed.down.dev_bytes : nullptr;
-        P.r_b = nullptr;
-        P.s_a = shared.present ? (const uint8_t*)shared.down.dev_bytes : nullptr;
-        P.s_b = nullptr;
+        const int qrd = routed.present ? routed.down.quant : shared.down.quant;
+        const int qsd = shared.present ? shared.down.quant : qrd;
         P.rows = (int)g.hidden; P.k = (int)g.intermediate;
         P.x_routed = m->inter_routed; P.x_shared = m->inter_shared;
-        P.row_tiles = (int)g.hidden / kPfTileM;
-        const size_t smem_dn = pf_smem(qrd, qsd);
-        if (wide) {
-            P.tm_routed = m->tm_routed_dn;
-            P.tm_shared = m->tm_shared_dn;
+        P.row_units = (int)g.hidden / (2 * kPfTileM);
+        if (routed.present) rcp = make_prefill_map(&P.tm_r_a, routed.down.dev_bytes, E * g.hidden, P.k, qrd);
+        if (!rcp && shared.present) rcp = make_prefill_map(&P.tm_s_a, shared.down.dev_bytes, g.hidden, P.k, qsd);
+        if (rcp) return rcp;
+        if (dense && !routed.present && (((uintptr_t)dense->residual | (uintptr_t)dense->l_out) & 15) == 0) {
+            P.residual = dense->residual;
+            P.l_out = dense->l_out;
+            dense->done = true;
         }
-        return launch_prefill<MODE_DOWN>(st, P, pf_grid, smem_dn, qrd, qsd, wide);
+        return launch_prefill<MODE_DOWN>(m, st, P, qrd, qsd);
     }
     StreamLaunch SL{};
     SL.top_k = L.top_k;
@@ -823,30 +794,6 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
     if (smem > 220 * 1024)
         return fail(XABE_ERR_UNSUPPORTED_GEOMETRY, "down row tile of %zu bytes does not fit shared memory", smem);
     return DISPATCH_QQ(launch_down, qr, qs, m, st, L, routed_blocks + shared_tiles, smem);
-}
-
-// What k_prefill_gemm_wide needs beyond the other kernels: the activations in dispatch order and the
-// tensor maps of its four activation sources, all handle-owned, made once.  Set-up time only (allocates).
-int setup_wide_prefill(xabe_moe* m) {
-    const size_t T = m->g.max_tokens, H = m->g.hidden, I = m->g.intermediate;
-    if (H % kSpanElems != 0 || I % kSpanElems != 0) {
-        m->pf_item_cols = kPfTileN;
-        return XABE_OK;
-    }
-    if (m->scope == XABE_SCOPE_ROUTED && !m->x_sorted) {
-        cudaError_t e = dev_alloc(&m->x_sorted, (size_t)m->sorted_capacity * H);
-        if (e != cudaSuccess)
-            return fail(XABE_ERR_DRIVER, "CUDA driver error: %s (allocating the permuted activations)",
-                        cudaGetErrorString(e));
-    }
-    int rc = make_rows_map(&m->tm_shared_gu, m->normed_h, T, H);
-    if (!rc) rc = make_rows_map(&m->tm_shared_dn, m->inter_shared, T, I);
-    if (!rc && m->scope == XABE_SCOPE_ROUTED) {
-        rc = make_rows_map(&m->tm_routed_gu, m->x_sorted, m->sorted_capacity, H);
-        if (!rc) rc = make_rows_map(&m->tm_routed_dn, m->inter_routed, m->sorted_capacity, I);
-    }
-    if (!rc) m->pf_item_cols = kPfWideItemCols;
-    return rc;
 }
 
 int check_routed(xabe_moe* m, const char* entry) {
@@ -982,7 +929,7 @@ int launch_route_and_dispatch(xabe_moe* m, cudaStream_t st, const float* logits)
         if (prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate)) {  // few experts, many tokens
             int threads = ((int)g.num_experts + 31) / 32 * 32;
             k_build_prefill_items<<<1, threads, hist_bytes, counted(st)>>>((int)g.num_experts, m->expert_offsets,
-                                                                  m->expert_counts, m->pf_items, m->pf_n_items, m->pf_item_cols);
+                                                                  m->expert_counts, m->pf_items, m->pf_n_items, kPfTileN);
             CUDA_TRY(cudaGetLastError());
         }
         return XABE_OK;
@@ -1010,7 +957,7 @@ int launch_route_and_dispatch(xabe_moe* m, cudaStream_t st, const float* logits)
     // Only the work list of the kernels that will run: the regime must be chosen before this call.
     if (prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate)) {
         k_build_prefill_items<<<1, threads, hist_bytes, counted(st)>>>((int)g.num_experts, m->expert_offsets,
-                                                              m->expert_counts, m->pf_items, m->pf_n_items, m->pf_item_cols);
+                                                              m->expert_counts, m->pf_items, m->pf_n_items, kPfTileN);
     } else {
         k_build_work<<<1, threads, hist_bytes, counted(st)>>>((int)g.num_experts, m->expert_offsets, m->expert_counts,
                                                      m->sorted_token_ids, m->topk_weights, m->work_items,
@@ -1172,13 +1119,6 @@ int xabe_moe_create(const xabe_moe_geometry* geometry, int device, int scope, fl
     xabe_moe* m = new (std::nothrow) xabe_moe();
     if (!m) return fail(XABE_ERR_DRIVER, "out of host memory");
     m->sm_count = prop.multiProcessorCount;
-    // Items of up to 512 token columns (four accumulators per unpacked weight pair, B tiles by TMA):
-    // measured faster only where every item is full and the contraction is long -- the dense block at
-    // prefill width (3.40 vs 3.77 ms per layer at 4096 tokens); with the routed experts the extra
-    // pass that permutes the activations costs more than the shared unpack work returns.
-    // XABE_TUNE_PREFILL_WIDE overrides the choice after creation.
-    m->pf_item_cols = (scope == XABE_SCOPE_SHARED_ONLY && g.max_tokens >= kPrefillWideMinTokens) ? kPfWideItemCols
-                                                                                                 : kPfTileN;
     m->g = g;
     m->device = device;
     m->scope = scope;
@@ -1242,13 +1182,6 @@ int xabe_moe_create(const xabe_moe_geometry* geometry, int device, int scope, fl
         xabe_moe_destroy(m);
         return fail(XABE_ERR_DRIVER, "CUDA driver error: %s (allocating MoE buffers)", cudaGetErrorString(e));
     }
-    if (m->pf_item_cols > kPfTileN) {
-        int rc = setup_wide_prefill(m);
-        if (rc) {
-            xabe_moe_destroy(m);
-            return rc;
-        }
-    }
     *out = m;
     return XABE_OK;
 }
@@ -1259,7 +1192,7 @@ void xabe_moe_destroy(xabe_moe* m) {
     void* dev[] = {m->valid_tokens, m->status, m->topk_ids, m->topk_weights, m->sorted_token_ids, m->expert_ids,
                    m->num_tokens_post_pad, m->chunk_hist, m->expert_offsets, m->expert_counts, m->front_tickets, m->tail_done, m->ep_compact, m->ep_rank_start, m->ep_send_counts, m->work_items, m->n_work, m->pf_items,
                    m->pf_n_items, m->normed, m->normed_h, m->logits,
-                   m->inter_routed, m->inter_shared, m->x_sorted, m->dense_partial, m->partial, m->routed, m->shexp, m->gate, m->stage_in,
+                   m->inter_routed, m->inter_shared, m->dense_partial, m->partial, m->routed, m->shexp, m->gate, m->stage_in,
                    m->stage_ffn, m->stage_out};
     for (void* p : dev)
         if (p) cudaFree(p);
@@ -1858,18 +1791,7 @@ int xabe_moe_set_tuning(xabe_moe* m, int key, int value) {
             m->fused_front = (value & 2) != 0;
             m->fused_norm = (value & 4) != 0;
             return XABE_OK;
-        case XABE_TUNE_PREFILL_WIDE:
-            if (value == 0) {
-                m->pf_item_cols = kPfTileN;
-                return XABE_OK;
-            }
-            {
-                const int rc = setup_wide_prefill(m);
-                // 2, 3: items of two or three 128-column tiles (the B ring then runs further ahead of the MMAs)
-                if (!rc && m->pf_item_cols > kPfTileN && value >= 2 && value < kPfWideMaxCt)
-                    m->pf_item_cols = value * kPfTileN;
-                return rc;
-            }
+        case XABE_TUNE_PREFILL_WIDE: return XABE_OK;  // one prefill kernel serves every width
         default: return fail(XABE_ERR_INVALID_ARGUMENT, "unknown tuning key %d", key);
     }
 }
