@@ -104,6 +104,21 @@ __device__ __forceinline__ void mma_f16_16816_acc(float (&d)[4], const uint32_t 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
 
+// silu(g) * u = g / (1 + expf(-g)) * u without a branch, so that a thread's outputs overlap (a division
+// that may leave for a slow path serialises them: 230 clocks each in a warp that had sixteen to do).  The
+// quotient is formed as Markstein (IBM J. Res. Dev. 34, 1990) shows for machines with fused multiply-add:
+// a Newton step on an approximate reciprocal, then one correction of the quotient by its exact remainder,
+// which rounds correctly for a divisor in [1, 2^126).  The exponent is clamped to stay there: below
+// g = -87 the true result is under 1e-35, zero in the f16 it is stored in.
+__device__ __forceinline__ float swiglu_fast(float g, float u) {
+    const float d = 1.0f + expf(fminf(-g, 87.0f));
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = fmaf(fmaf(-d, r, 1.0f), r, r);
+    const float q = g * r, q2 = fmaf(fmaf(-q, d, g), r, q);
+    return (q2 == q2 ? q2 : q) * u;  // (an infinite g has no remainder)
+}
+
 // 32-bit word at a 2-byte-aligned shared-memory address.
 __device__ __forceinline__ uint32_t ld32_al2(const uint8_t* p) {
     uintptr_t a = (uintptr_t)p;

@@ -16,8 +16,11 @@
 //     tcgen05.st into a ring of four A stages in tensor memory (128 rows x 128
 //     contraction elements each).  One scale serves the sixteen weights of a
 //     store, and the weights never pass through shared memory;
-//   * two warps gather the token rows of the tile (B operand) with 16-byte
-//     asynchronous copies into 128-byte-swizzled shared-memory tiles;
+//   * two warps bring the token rows of the tile (B operand) into 128-byte-swizzled
+//     shared-memory tiles: rows that lie one after the other (the down projection's
+//     slots, the shared expert's tokens) with TMA boxes of 32 rows, a routed gate/up
+//     tile's scattered rows with 16-byte asynchronous copies (tile::gather4 was
+//     measured: 97 clocks per four rows, 1.6 times the whole launch's time);
 //   * one thread issues tcgen05.mma (A from tensor memory, M128 K16, N = the
 //     tile's token count rounded up to 16);
 //   * four epilogue warps read finished accumulators (a thread = a weight row,
@@ -64,11 +67,12 @@ constexpr int kPfUnpackWarps = 16;
 constexpr int kPfWarpEpi0 = 16;     // four epilogue warps; warp % 4 is the lane quadrant a warp may touch
 constexpr int kPfWarpMma = 20;
 constexpr int kPfWarpRaw = 21;
-constexpr int kPfWarpLoad = 22;     // two B loader warps
+constexpr int kPfWarpLoad = 22;     // token rows: two warps
 constexpr int kPfLoadWarps = 2;
 constexpr int kPfThreads = 32 * 24;
-constexpr int kPfAStages = 4;       // half a span x two row tiles
-constexpr int kPfRawSlots = 16;     // two spans x two row tiles x four quadrants of 32 rows
+constexpr int kPfAStages = 2;       // half a span of both row tiles each
+constexpr int kPfRawSlots = 2;      // one span of both row tiles each
+constexpr int kPfBoxTokens = 32;    // token rows of one box where they lie one after the other
 constexpr int kPfMaxBStages = 5;
 constexpr int kPfEpiTokens = 16;    // tokens the epilogue turns around at a time
 constexpr int kPfEpiBytes = kPfEpiTokens * kPfTileM * 4;  // 8 KB, two of them
@@ -79,13 +83,16 @@ constexpr int kPfItemInts = 4;  // expert, first slot (or first token), columns,
 // Weight rows as the TMA reads them.  A row's bytes are a multiple of 2 only (210 per Q6_K superblock), a
 // tensor map's pitch must be one of 16: R = 1, 2, 4 or 8 neighbouring rows make one row of the map.
 // Rows r % R == c (class c) then start at byte c * row_bytes of it and share one 16-byte alignment.
-// Slot s of a 128-row tile (lane s % 32 of quadrant s / 32) holds row (s % (128 / R)) * R + s / (128 / R),
-// so the 32 rows of a quadrant are of one class (R <= 4; of two for R = 8, whose boxes are 16 rows high).
+// Slot s of a 128-row tile (lane s % 32 of quadrant s / 32) holds row (s % (128 / R)) * R + s / (128 / R):
+// a class is one box of 128 / R rows, and the 32 rows of a quadrant are of one class (R <= 4; of two for
+// R = 8).
 __host__ __device__ inline int pf_row_group(uint32_t row_bytes) {
     return row_bytes % 16 == 0 ? 1 : row_bytes % 8 == 0 ? 2 : row_bytes % 4 == 0 ? 4 : 8;
 }
 
 struct PrefillLaunch {
+    CUtensorMap tm_x_r, tm_x_s;  // token rows ([rows][k] f16) of the down projection's slots and of the shared expert
+    const __half* x_routed;      // gate/up: normed_h [token]
     CUtensorMap tm_r_a, tm_r_b, tm_s_a, tm_s_b;  // weight bytes: routed gate (or down), routed up, shared gate (or down), shared up
     int rows;            // output rows per matrix
     int k;               // contraction length
@@ -96,8 +103,6 @@ struct PrefillLaunch {
     const int* valid_tokens;
     const int* sorted_token_ids;
     const float* topk_weights;
-    const __half* x_routed;  // gate/up: normed_h [token]; down: inter [slot]
-    const __half* x_shared;  // gate/up: normed_h [token]; down: inter_shared [token]
     __half* inter_routed;
     __half* inter_shared;
     float* partial;
@@ -108,7 +113,7 @@ struct PrefillLaunch {
     int* status;
     int row_units;   // tiles along the weight rows: gate/up rows / 128, down rows / 256
     int n_b;         // B stages
-    int slot_bytes;  // raw slot: 32 * the larger row pitch of the formats in this launch
+    int slot_bytes;  // raw slot: 256 * the larger row pitch of the formats in this launch
 };
 
 // ---- tcgen05 / TMEM wrappers ------------------------------------------------
@@ -163,8 +168,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// The registers of earlier loads may be read once this has returned (they are operands, so that no use of
+// them is scheduled above it).
+__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle:
@@ -193,6 +204,13 @@ __device__ __forceinline__ uint32_t swz_off(int row, int chunk) {
     return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
 }
 
+__device__ __forceinline__ void tma_load_box_2d32(uint32_t dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            dst),
+        "l"((uint64_t)tm), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
 // 16-byte asynchronous copy global -> shared (zero-filled when src_bytes is 0), and the arrival it
 // triggers on an mbarrier once all of this thread's earlier copies have landed.  The arrival does
 // not raise the barrier's pending count: the count it was initialised with includes it.
@@ -212,12 +230,15 @@ __device__ __forceinline__ void mbar_arrive32(uint32_t bar) {
 }
 
 // Bounded wait that also gives up when another warp of the CTA already has.  try_wait itself
-// suspends the thread for a hardware-defined slice, so the roles inside the per-pair pipeline poll
+// suspends the thread for a hardware-defined slice, so the roles inside the per-span pipeline poll
 // without sleeping (a sleeping waiter adds its sleep to every hand-over); only the epilogue warps,
-// which wait for a whole tile, back off.
+// which wait for a whole tile, back off.  The single-thread roles are paced by instruction fetch (the
+// unpack warps keep sweeping the nearest caches): the satisfied wait is the straight-line path, the loop
+// lies out of line.
 template <bool BACKOFF = false>
 __device__ __forceinline__ bool stream_wait_pf(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                int* status) {
+    if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
     for (uint32_t it = 0; it < kWaitLimit; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((it & 63u) == 63u && *abort_flag) return false;
@@ -226,6 +247,12 @@ __device__ __forceinline__ bool stream_wait_pf(uint64_t* bar, uint32_t parity, v
     *abort_flag = 1;
     if (status) atomicExch(status, STATUS_TMA_TIMEOUT);
     return false;
+}
+
+// The same for a whole converged warp, with one verdict.
+template <bool BACKOFF = false>
+__device__ __forceinline__ bool warp_wait_pf(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+    return __all_sync(0xffffffffu, stream_wait_pf<BACKOFF>(bar, parity, abort_flag, status));
 }
 
 // Token tiles of the routed experts for the prefill kernels: the live slots of
@@ -399,10 +426,10 @@ __device__ __forceinline__ void pf_unpack8(const uint32_t (&a)[36], uint32_t tad
 // Shared-memory control block of the kernel.
 struct PfCtl {
     uint64_t raw_full[kPfRawSlots];   // TMA bytes landed -> unpack warps
-    uint64_t raw_empty[kPfRawSlots];  // two unpack warps (the halves of the span) -> TMA thread
-    uint64_t a_full[kPfAStages];      // four unpack warps -> MMA
+    uint64_t raw_empty[kPfRawSlots];  // unpack warps -> TMA thread
+    uint64_t a_full[kPfAStages];      // the eight unpack warps of a half -> MMA
     uint64_t a_empty[kPfAStages];     // MMA (tcgen05.commit) -> unpack warps
-    uint64_t b_full[kPfMaxBStages];   // every B loader lane's copies landed -> MMA
+    uint64_t b_full[kPfMaxBStages];   // every loader lane (its copies landed) -> MMA
     uint64_t b_empty[kPfMaxBStages];  // MMA (tcgen05.commit) -> B loaders
     uint64_t acc_full[2];             // MMA (tcgen05.commit) -> epilogue, by tile parity
     uint64_t acc_empty[2];            // epilogue -> MMA, by half of the accumulator columns
@@ -452,10 +479,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
         ctl.abort_flag = 0;
         for (int i = 0; i < kPfRawSlots; ++i) {
             mbar_init(&ctl.raw_full[i], 1);
-            mbar_init(&ctl.raw_empty[i], 2);
+            mbar_init(&ctl.raw_empty[i], kPfUnpackWarps);
         }
         for (int i = 0; i < kPfAStages; ++i) {
-            mbar_init(&ctl.a_full[i], 4);
+            mbar_init(&ctl.a_full[i], kPfUnpackWarps / 2);
             mbar_init(&ctl.a_empty[i], 1);
         }
         for (int i = 0; i < NB; ++i) {
@@ -479,10 +506,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
 
     if (warp < kPfUnpackWarps) {
         // ------------------------------ unpack warps ------------------------------
-        // Warp 4 i + q: quadrant q (slots 32 q .. 32 q + 31) of row tile i % 2, half i / 2 of every span,
-        // i.e. A stage i.
-        const int q = warp & 3, stage = warp >> 2, rt = stage & 1, h = stage >> 1;
-        const uint32_t taddr = tmem_base + kPfColsA + (uint32_t)stage * 64u + ((uint32_t)(q * 32) << 16);
+        // Warp 8 h + 4 rt + q: quadrant q (slots 32 q .. 32 q + 31) of row tile rt, half h of every span,
+        // which is also the A stage.
+        const int q = warp & 3, rt = (warp >> 2) & 1, h = warp >> 3;
+        const uint32_t taddr = tmem_base + kPfColsA + (uint32_t)(h * 2 + rt) * 64u + ((uint32_t)(q * 32) << 16);
         uint32_t n = 0;  // spans since the kernel started
         bool ok = true;
         PfTile T{}, T1{};
@@ -494,19 +521,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
             const int row_b = n_spans * span_b, R = pf_row_group((uint32_t)row_b);
             const int cls = (32 * q + lane) / (kPfTileM / R);
             for (int s = 0; s < n_spans; ++s, ++n) {
-                const int slot = (int)(n & 1) * 8 + rt * 4 + q;
-                ok = __all_sync(0xffffffffu,
-                                stream_wait_pf(&ctl.raw_full[slot], (n >> 1) & 1, abortp, L.status));
+                const int slot = (int)(n & 1);
+                ok = warp_wait_pf(&ctl.raw_full[slot], (n >> 1) & 1, abortp, L.status);
                 if (!ok) break;
                 const int x = cls * row_b + s * span_b;
                 const uint32_t delta = (uint32_t)(x - rows_box_start(x, R * row_b, box));
-                const uint32_t gb = raw32 + (uint32_t)(slot * L.slot_bytes + lane * box) + (delta & ~15u);
-                auto stage_free = [&]() -> bool {  // the bytes are in registers: hand the raw slot back, wait for the stage
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive32(smem_u32(&ctl.raw_empty[slot]));
+                const uint32_t gb = raw32 + (uint32_t)(slot * L.slot_bytes + (rt * kPfTileM + q * 32 + lane) * box) + (delta & ~15u);
+                auto stage_free = [&]() -> bool {
                     bool o = true;
-                    if (n >= 1) o = stream_wait_pf(&ctl.a_empty[stage], (n - 1) & 1, abortp, L.status);
-                    o = __all_sync(0xffffffffu, o);
+                    if (n >= 1) o = warp_wait_pf(&ctl.a_empty[h], (n - 1) & 1, abortp, L.status);
                     tc_fence_after();
                     return o;
                 };
@@ -533,7 +556,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive32(smem_u32(&ctl.a_full[stage]));
+                if (lane == 0) {
+                    mbar_arrive32(smem_u32(&ctl.a_full[h]));
+                    // Only here is it certain that the raw bytes have been read: an arrival right behind the
+                    // shared loads (whose results nothing had used yet) let the next span's copy overtake them.
+                    mbar_arrive32(smem_u32(&ctl.raw_empty[slot]));
+                }
             }
             T = T1;
         }
@@ -566,7 +594,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                 ctl.dst[tp][etid] = p;
                 ctl.factor[tp][etid] = f;
             }
-            bool ok = stream_wait_pf<true>(&ctl.acc_full[tp], (n >> 1) & 1, abortp, L.status);
+            bool ok = warp_wait_pf<true>(&ctl.acc_full[tp], (n >> 1) & 1, abortp, L.status);
             ok = pf_epi_agree(ok);
             if (!ok) break;
             tc_fence_after();
@@ -591,27 +619,27 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                     if (MODE == MODE_GATEUP) {
                         uint32_t u[16];
                         tmem_ld16(tq + (uint32_t)(128 + st * kPfEpiTokens), u);
-                        tmem_ld_wait();
+                        tmem_ld_wait16(r);
+                        tmem_ld_wait16(u);
                         if (st == steps - 1) release();
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const float gv = __uint_as_float(r[i]) * inv, uv = __uint_as_float(u[i]) * inv;
-                            buf[i * kPfTileM + lslot] = __fdiv_rn(gv, 1.0f + expf(-gv)) * uv;
+                            buf[i * kPfTileM + lslot] = swiglu_fast(gv, uv);
                         }
                     } else {
-                        tmem_ld_wait();
+                        tmem_ld_wait16(r);
                         if (rt == RTS - 1 && st == steps - 1) release();
 #pragma unroll
                         for (int i = 0; i < 16; ++i) buf[i * kPfTileM + lslot] = __uint_as_float(r[i]);
                     }
                     asm volatile("bar.sync 2, 128;" ::: "memory");  // the four epilogue warps
                     // (the other buffer is rewritten only after every warp has passed the next barrier)
+                    float4 w[4];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const int row = quad * 4 + k, tok = st * kPfEpiTokens + row;
-                        if (tok >= T.ncols) break;
-                        const float* src = buf + row * kPfTileM;
-                        float4 v;
+                        const float* src = buf + (quad * 4 + k) * kPfTileM;
+                        float4& v = w[k];
                         if (R == 1) {
                             v = *(const float4*)(src + 4 * lane);
                         } else if (R == 2) {
@@ -623,6 +651,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                             const float* p = src + (lane & 1) * 64 + (lane >> 1);
                             v = make_float4(p[0], p[16], p[32], p[48]);
                         }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int tok = st * kPfEpiTokens + quad * 4 + k;
+                        if (tok >= T.ncols) break;
+                        float4 v = w[k];
                         if (MODE == MODE_GATEUP) {
                             const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
                             __half* dst = (T.shared ? L.inter_shared : L.inter_routed) + (size_t)(T.first + tok) * L.rows +
@@ -677,42 +711,37 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                 tc_fence_after();
                 const uint32_t d0 = tmem_base + half * 64u;
                 for (int s = 0; s < n_spans && ok; ++s, ++n) {
-#pragma unroll 1
-                    for (int h = 0; h < 2 && ok; ++h) {
-                        int st[2];
-                        uint32_t baddr[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {  // straight-line code for the whole span
+                        if (!stream_wait_pf(&ctl.a_full[h], n & 1, abortp, L.status)) {
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t ta = tmem_base + kPfColsA + (uint32_t)h * 128u;
 #pragma unroll
                         for (int c = 0; c < 2; ++c) {
-                            if (ok) ok = stream_wait_pf(&ctl.b_full[bs], bph, abortp, L.status);
-                            st[c] = bs;
-                            baddr[c] = smem_u32(bst) + (uint32_t)bs * kPfBStageBytes;
+                            if (!stream_wait_pf(&ctl.b_full[bs], bph, abortp, L.status)) {
+                                ok = false;
+                                break;
+                            }
+                            tc_fence_after();
+                            if (MODE == MODE_GATEUP) fence_proxy_async_smem();  // rows that arrived by cp.async
+                            const uint64_t xdesc = umma_smem_desc(smem_u32(bst) + (uint32_t)bs * kPfBStageBytes);
+                            const uint32_t tc = ta + (uint32_t)c * 32u;
+#pragma unroll
+                            for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+                                for (int k4 = 0; k4 < 4; ++k4)  // 32 bytes per K16 step inside the swizzle row
+                                    umma_f16_ta(d0 + (uint32_t)rt * 128u, tc + (uint32_t)(rt * 64 + k4 * 8), xdesc + 2 * k4,
+                                                idesc, (s > 0 || h > 0 || c > 0 || k4 > 0) ? 1u : 0u);
+                            umma_commit(&ctl.b_empty[bs]);
                             if (++bs == NB) {
                                 bs = 0;
                                 bph ^= 1u;
                             }
                         }
                         if (!ok) break;
-                        fence_proxy_async_smem();  // the B tiles arrived by cp.async, not through the async proxy
-#pragma unroll 1
-                        for (int rt = 0; rt < 2; ++rt) {
-                            const int as = h * 2 + rt;
-                            ok = stream_wait_pf(&ctl.a_full[as], n & 1, abortp, L.status);
-                            if (!ok) break;
-                            tc_fence_after();
-                            const uint32_t ta = tmem_base + kPfColsA + (uint32_t)as * 64u, td = d0 + (uint32_t)rt * 128u;
-#pragma unroll
-                            for (int c = 0; c < 2; ++c) {
-                                const uint64_t xdesc = umma_smem_desc(baddr[c]);
-#pragma unroll
-                                for (int k4 = 0; k4 < 4; ++k4)  // 32 bytes per K16 step inside the swizzle row
-                                    umma_f16_ta(td, ta + (uint32_t)((c * 4 + k4) * 8), xdesc + 2 * k4, idesc,
-                                                (s > 0 || h > 0 || c > 0 || k4 > 0) ? 1u : 0u);
-                            }
-                            umma_commit(&ctl.a_empty[as]);
-                        }
-                        if (!ok) break;
-                        umma_commit(&ctl.b_empty[st[0]]);
-                        umma_commit(&ctl.b_empty[st[1]]);
+                        umma_commit(&ctl.a_empty[h]);
                     }
                 }
                 if (ok) umma_commit(&ctl.acc_full[tn & 1]);
@@ -731,24 +760,22 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                 const int quant = T.shared ? QS : QR;
                 const int span_b = span_bytes_of(quant), box = (int)rows_box_bytes(quant);
                 const int row_b = n_spans * span_b, R = pf_row_group((uint32_t)row_b);
-                const int per_class = kPfTileM / R, box_rows = per_class < 32 ? per_class : 32;
+                const int per_class = kPfTileM / R;
                 const int row0 = T.expert * L.rows + T.bx * (MODE == MODE_GATEUP ? kPfTileM : 2 * kPfTileM);
-                for (int s = 0; s < n_spans && ok; ++s, ++n) {
-                    for (int i = 0; i < 8 && ok; ++i) {
-                        const int rt = i >> 2, q = i & 3, slot = (int)(n & 1) * 8 + i;
-                        if (n >= 2) ok = stream_wait_pf(&ctl.raw_empty[slot], ((n >> 1) - 1) & 1, abortp, L.status);
-                        if (!ok) break;
-                        const CUtensorMap* tm = MODE == MODE_GATEUP && rt == 1 ? (T.shared ? &L.tm_s_b : &L.tm_r_b)
-                                                                               : (T.shared ? &L.tm_s_a : &L.tm_r_a);
-                        const int rows_at = row0 + (MODE == MODE_DOWN ? rt * kPfTileM : 0);
-                        uint8_t* dst = smem_raw + (raw32 - smem_u32(smem_raw)) + (size_t)slot * L.slot_bytes;
-                        mbar_expect_tx(&ctl.raw_full[slot], 32u * (uint32_t)box);
-                        for (int b = 0; b < 32; b += box_rows) {
-                            const int sl = 32 * q + b, cls = sl / per_class;
-                            const int x = rows_box_start(cls * row_b + s * span_b, R * row_b, box);
-                            tma_load_box_2d(dst + b * box, tm, x >> 2, rows_at / R + sl - cls * per_class,
-                                            &ctl.raw_full[slot]);
-                        }
+                const CUtensorMap* tm0 = T.shared ? &L.tm_s_a : &L.tm_r_a;
+                const CUtensorMap* tm1 = MODE == MODE_GATEUP ? (T.shared ? &L.tm_s_b : &L.tm_r_b) : tm0;
+                const int y0 = row0 / R, y1 = (row0 + (MODE == MODE_GATEUP ? 0 : kPfTileM)) / R;
+                for (int s = 0; s < n_spans; ++s, ++n) {
+                    const int slot = (int)(n & 1);
+                    if (n >= 2) ok = stream_wait_pf(&ctl.raw_empty[slot], ((n >> 1) - 1) & 1, abortp, L.status);
+                    if (!ok) break;
+                    uint8_t* dst = smem_raw + (raw32 - smem_u32(smem_raw)) + (size_t)slot * L.slot_bytes;
+                    mbar_expect_tx(&ctl.raw_full[slot], 2u * kPfTileM * (uint32_t)box);
+#pragma unroll 1
+                    for (int cls = 0; cls < R; ++cls, dst += per_class * box) {
+                        const int x = rows_box_start(cls * row_b + s * span_b, R * row_b, box) >> 2;
+                        tma_load_box_2d(dst, tm0, x, y0, &ctl.raw_full[slot]);
+                        tma_load_box_2d(dst + kPfTileM * box, tm1, x, y1, &ctl.raw_full[slot]);
                     }
                 }
                 T = T1;
@@ -756,29 +783,30 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
             // after an abort: let the copies in flight land before the CTA's shared memory is handed on
             if (!ok)
                 for (uint32_t back = 0; back < 2 && back <= n; ++back)
-                    for (int i = 0; i < 8; ++i)
-                        for (uint32_t it = 0; it < 4096u; ++it)
-                            if (mbar_try_wait(&ctl.raw_full[((n - back) & 1) * 8 + i], ((n - back) >> 1) & 1)) break;
+                    for (uint32_t it = 0; it < kWaitLimit; ++it)
+                        if (mbar_try_wait(&ctl.raw_full[(n - back) & 1], ((n - back) >> 1) & 1)) break;
         }
     } else {
-        // ------------------------------ B loaders ------------------------------
-        // A pass of one warp covers four rows (eight lanes of 16 bytes each); lane's rows are
-        // 8 i + 4 lw + lane / 8, i = 0 .. 15.
+        // ------------------------------ token rows ------------------------------
+        // Scattered rows: a pass of one warp covers four rows (eight lanes of 16 bytes each); a lane's rows
+        // are 8 i + 4 lw + lane / 8, i = 0 .. 15.
         const int lw = warp - kPfWarpLoad, piece = lane & 7, rlow = 4 * lw + (lane >> 3);
-        const uint32_t doff = smem_u32(bst) + swz_off(rlow, piece);
+        const uint32_t b32 = smem_u32(bst), doff = b32 + swz_off(rlow, piece);
         int bs = 0;
-        uint32_t bph = 0;
-        bool ok = true, wrapped = false;
+        uint32_t bph = 0, issued = 0;
+        bool ok = true;
         auto token_rows = [&](const PfTile& T, int (&xo)[16]) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int c = 8 * i + rlow;
-                int src = -1;
-                if (c < T.ncols) {
-                    if (T.shared || MODE == MODE_DOWN) src = T.first + c;
-                    else src = __ldg(L.sorted_token_ids + T.first + c) / L.top_k;
-                }
-                xo[i] = src;
+                xo[i] = !T.shared && c < T.ncols ? __ldg(L.sorted_token_ids + T.first + c) / L.top_k : -1;
+            }
+        };
+        auto advance = [&]() {
+            ++issued;
+            if (++bs == NB) {
+                bs = 0;
+                bph ^= 1u;
             }
         };
         // the tile record runs two tiles ahead of the work, the token rows one
@@ -786,36 +814,63 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
         int xr[16], xr1[16];
         if ((int)blockIdx.x < n_tiles) {
             T = pf_tile(L, blockIdx.x, n_routed, valid);
-            token_rows(T, xr);
+            if (MODE == MODE_GATEUP) token_rows(T, xr);
         }
         if ((int)blockIdx.x + G < n_tiles) T1 = pf_tile(L, blockIdx.x + G, n_routed, valid);
         for (int t = blockIdx.x; t < n_tiles && ok; t += G) {
-            if (t + G < n_tiles) token_rows(T1, xr1);
+            if (MODE == MODE_GATEUP && t + G < n_tiles) token_rows(T1, xr1);
             if (t + 2 * G < n_tiles) T2 = pf_tile(L, t + 2 * G, n_routed, valid);
-            const uint8_t* xb = (const uint8_t*)(T.shared ? L.x_shared : L.x_routed) + piece * 16;
-            const size_t pitch = (size_t)L.k * 2;
-            for (int c = 0; c < L.k / kPfChunkK && ok; ++c, xb += 2 * kPfChunkK) {
-                if (wrapped) {
-                    ok = stream_wait_pf(&ctl.b_empty[bs], bph ^ 1u, abortp, L.status);
-                    if (!ok) break;
-                }
-                const uint32_t dst = doff + (uint32_t)bs * kPfBStageBytes;
+            if (MODE == MODE_GATEUP && !T.shared) {
+                const uint8_t* xb = (const uint8_t*)L.x_routed + piece * 16;
+                const size_t pitch = (size_t)L.k * 2;
+                for (int c = 0; c < L.k / kPfChunkK; ++c, xb += 2 * kPfChunkK) {
+                    if (issued >= (uint32_t)NB) {
+                        ok = warp_wait_pf(&ctl.b_empty[bs], bph ^ 1u, abortp, L.status);
+                        if (!ok) break;
+                    }
+                    const uint32_t dst = doff + (uint32_t)bs * kPfBStageBytes;
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (xr[i] >= 0) cp_async16(dst + i * 1024u, xb + (size_t)xr[i] * pitch, 16u);
-                cp_async_arrive_noinc(&ctl.b_full[bs]);
-                if (++bs == NB) {
-                    bs = 0;
-                    bph ^= 1u;
-                    wrapped = true;
+                    for (int i = 0; i < 16; ++i)
+                        if (xr[i] >= 0) cp_async16(dst + i * 1024u, xb + (size_t)xr[i] * pitch, 16u);
+                    cp_async_arrive_noinc(&ctl.b_full[bs]);
+                    advance();
+                }
+            } else {
+                const CUtensorMap* tm = T.shared ? &L.tm_x_s : &L.tm_x_r;
+                const int boxes = (T.ncols + kPfBoxTokens - 1) / kPfBoxTokens;
+                for (int c = 0; c < L.k / kPfChunkK; ++c) {
+                    if (issued >= (uint32_t)NB) {
+                        ok = warp_wait_pf(&ctl.b_empty[bs], bph ^ 1u, abortp, L.status);
+                        if (!ok) break;
+                    }
+                    uint64_t* full = &ctl.b_full[bs];
+                    if (lw == 0 && lane == 0) mbar_expect_tx(full, (uint32_t)boxes * kPfBoxTokens * kPfChunkK * 2u);
+                    else mbar_arrive32(smem_u32(full));
+                    __syncwarp();
+                    if (lw == 0 && lane < boxes)
+                        tma_load_box_2d32(b32 + (uint32_t)bs * kPfBStageBytes + (uint32_t)lane * (kPfBoxTokens * 128u), tm,
+                                          c * kPfChunkK, T.first + lane * kPfBoxTokens, full);
+                    advance();
                 }
             }
             T = T1;
             T1 = T2;
+            if (MODE == MODE_GATEUP) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) xr[i] = xr1[i];
+                for (int i = 0; i < 16; ++i) xr[i] = xr1[i];
+            }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
+        // after an abort: let the boxes in flight land before the CTA's shared memory is handed on
+        if (!ok)
+            for (uint32_t back = 0; back < (uint32_t)NB && back < issued; ++back) {
+                if (--bs < 0) {
+                    bs = NB - 1;
+                    bph ^= 1u;
+                }
+                for (uint32_t it = 0; it < kWaitLimit; ++it)
+                    if (mbar_try_wait(&ctl.b_full[bs], bph)) break;
+            }
     }
     // every thread of the CTA arrives here on every path, so tensor memory is always returned
     tc_fence_before();

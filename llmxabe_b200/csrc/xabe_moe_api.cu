@@ -442,13 +442,31 @@ bool prefill_applies(const xabe_moe* m, int gateup_rows, int down_rows, int hidd
     return m->g.max_tokens >= kPrefillMinTokens;
 }
 
+// The tensor map k_prefill_gemm reads token rows ([rows][k] f16) through: 64 elements x `box_rows` rows,
+// 128-byte swizzle, rows out of bounds read as zero.
+int make_rows_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    if (!enc) return fail(XABE_ERR_DRIVER, "cuTensorMapEncodeTiled is not available from this driver");
+    if (((uintptr_t)base & 15) != 0 || k % 64 != 0 || rows == 0)
+        return fail(XABE_ERR_INVALID_ARGUMENT, "tensor map source must be 16-byte aligned with k a multiple of 64");
+    cuuint64_t dims[2] = {k, rows};
+    cuuint64_t strides[1] = {k * 2};
+    cuuint32_t box[2] = {(cuuint32_t)kPfChunkK, box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(XABE_ERR_DRIVER, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return XABE_OK;
+}
+
 // The tensor map k_prefill_gemm reads a weight stack of `rows` rows of `k` elements through.
 int make_prefill_map(CUtensorMap* out, const void* base, uint64_t rows, int k, int quant) {
     const int q = quant == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0;
     const uint32_t row_bytes = (uint32_t)(k / kSpanElems * span_bytes_of(q));
     const int R = pf_row_group(row_bytes);
     return make_bytes_map(out, base, rows / R, (uint64_t)row_bytes * R, rows_box_bytes(q),
-                          (uint32_t)std::min(32, kPfTileM / R));
+                          (uint32_t)(kPfTileM / R));
 }
 
 template <int MODE, int QR, int QS>
@@ -465,7 +483,7 @@ int launch_prefill(xabe_moe* m, cudaStream_t st, PrefillLaunch& L, int qr, int q
     int box = 0;
     if (L.has_routed) box = (int)rows_box_bytes(qr == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
     if (L.has_shared) box = std::max(box, (int)rows_box_bytes(qs == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0));
-    L.slot_bytes = 32 * box;
+    L.slot_bytes = 2 * kPfTileM * box;
     L.n_b = kPfMaxBStages;
     while (L.n_b > 2 && pf_smem_bytes(L.slot_bytes, L.n_b) > 223u * 1024u) --L.n_b;
     const uint32_t smem = pf_smem_bytes(L.slot_bytes, L.n_b);
@@ -660,16 +678,17 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
         P.shexp = shexp_out;
         P.status = m->status;
         P.rows = (int)g.intermediate; P.k = (int)g.hidden;
-        P.x_routed = x_routed; P.x_shared = m->normed_h;
         P.row_units = (int)g.intermediate / kPfTileM;
         const uint64_t E = g.num_experts;
         int rcp = XABE_OK;
+        P.x_routed = x_routed;
         if (routed.present) {
             rcp = make_prefill_map(&P.tm_r_a, L.r_a, E * g.intermediate, P.k, qr);
             if (!rcp) rcp = make_prefill_map(&P.tm_r_b, L.r_b, E * g.intermediate, P.k, qr);
         }
         if (!rcp && shared.present) {
-            rcp = make_prefill_map(&P.tm_s_a, L.s_a, g.intermediate, P.k, qs);
+            rcp = make_rows_map(&P.tm_x_s, m->normed_h, g.max_tokens, P.k, kPfBoxTokens);
+            if (!rcp) rcp = make_prefill_map(&P.tm_s_a, L.s_a, g.intermediate, P.k, qs);
             if (!rcp) rcp = make_prefill_map(&P.tm_s_b, L.s_b, g.intermediate, P.k, qs);
         }
         if (!rcp) rcp = launch_prefill<MODE_GATEUP>(m, st, P, qr, qs);
@@ -678,10 +697,15 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
         const int qrd = routed.present ? routed.down.quant : shared.down.quant;
         const int qsd = shared.present ? shared.down.quant : qrd;
         P.rows = (int)g.hidden; P.k = (int)g.intermediate;
-        P.x_routed = m->inter_routed; P.x_shared = m->inter_shared;
         P.row_units = (int)g.hidden / (2 * kPfTileM);
-        if (routed.present) rcp = make_prefill_map(&P.tm_r_a, routed.down.dev_bytes, E * g.hidden, P.k, qrd);
-        if (!rcp && shared.present) rcp = make_prefill_map(&P.tm_s_a, shared.down.dev_bytes, g.hidden, P.k, qsd);
+        if (routed.present) {
+            rcp = make_rows_map(&P.tm_x_r, m->inter_routed, m->sorted_capacity, P.k, kPfBoxTokens);
+            if (!rcp) rcp = make_prefill_map(&P.tm_r_a, routed.down.dev_bytes, E * g.hidden, P.k, qrd);
+        }
+        if (!rcp && shared.present) {
+            rcp = make_rows_map(&P.tm_x_s, m->inter_shared, g.max_tokens, P.k, kPfBoxTokens);
+            if (!rcp) rcp = make_prefill_map(&P.tm_s_a, shared.down.dev_bytes, g.hidden, P.k, qsd);
+        }
         if (rcp) return rcp;
         if (dense && !routed.present && (((uintptr_t)dense->residual | (uintptr_t)dense->l_out) & 15) == 0) {
             P.residual = dense->residual;
