@@ -60,22 +60,21 @@ namespace xabe {
 
 constexpr int kPfTileM = 128;       // weight rows per row tile (tensor-memory lanes); a CTA's tile has two
 constexpr int kPfTileN = 128;       // token columns per tile
-constexpr int kPfChunkK = 64;       // contraction elements per B stage (one 128-byte swizzle row of f16)
-constexpr int kPfStageK = 128;      // contraction elements per A stage (half a span)
+constexpr int kPfChunkK = 64;       // contraction elements per stage (one 128-byte swizzle row of f16)
 constexpr int kPfBStageBytes = kPfTileN * kPfChunkK * 2;  // 16 KB
 constexpr int kPfUnpackWarps = 16;
-constexpr int kPfWarpEpi0 = 16;     // four epilogue warps; warp % 4 is the lane quadrant a warp may touch
-constexpr int kPfWarpMma = 20;
-constexpr int kPfWarpRaw = 21;
-constexpr int kPfWarpLoad = 22;     // token rows: two warps
+constexpr int kPfWarpEpi0 = 16;     // two teams of four epilogue warps; warp % 4 is the lane quadrant a warp may touch
+constexpr int kPfEpiTeams = 2;
+constexpr int kPfWarpMma = 24;
+constexpr int kPfWarpRaw = 25;
+constexpr int kPfWarpLoad = 26;     // token rows: two warps
 constexpr int kPfLoadWarps = 2;
-constexpr int kPfThreads = 32 * 24;
-constexpr int kPfAStages = 2;       // half a span of both row tiles each
+constexpr int kPfThreads = 32 * 28;
+constexpr int kPfStages = 4;        // one span: 64 contraction elements of both row tiles (A) and of the tokens (B) each
 constexpr int kPfRawSlots = 2;      // one span of both row tiles each
 constexpr int kPfBoxTokens = 32;    // token rows of one box where they lie one after the other
-constexpr int kPfMaxBStages = 5;
-constexpr int kPfEpiTokens = 16;    // tokens the epilogue turns around at a time
-constexpr int kPfEpiBytes = kPfEpiTokens * kPfTileM * 4;  // 8 KB, two of them
+constexpr int kPfEpiTokens = 16;    // tokens an epilogue team reads at a time
+constexpr int kPfEpiBytes = 4096;   // what it turns around at a time; two buffers per team
 constexpr uint32_t kPfColsA = 256;  // tensor-memory column of the first A stage (accumulators below it)
 constexpr float kPfWeightScale = 256.0f;
 constexpr int kPfItemInts = 4;  // expert, first slot (or first token), columns, pad
@@ -112,7 +111,6 @@ struct PrefillLaunch {
     float* l_out;
     int* status;
     int row_units;   // tiles along the weight rows: gate/up rows / 128, down rows / 256
-    int n_b;         // B stages
     int slot_bytes;  // raw slot: 256 * the larger row pitch of the formats in this launch
 };
 
@@ -369,29 +367,27 @@ __device__ __forceinline__ void pf_load6(uint32_t gb, uint32_t mm2, int h, PfHal
     H.d = __half2float(__ushort_as_half((unsigned short)t[4])) * kPfWeightScale;
 }
 // Element map of crates/xabe-kernels/src/quant.rs:175-198: group j (32 elements of the half), c = l / 16 is
-// contraction step 2 j + c of the half; its scale is number 2 j + c of the half's eight.
+// contraction step 2 j + c of the half; its scale is number 2 j + c of the half's eight.  Stage K of the
+// half: groups 2 K and 2 K + 1, the low (K = 0) or high nibbles of ql.
+template <int K>
 __device__ __forceinline__ void pf_unpack6(const PfHalf6& H, uint32_t taddr) {
     const uint32_t m = 0x0F0F0F0Fu;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        uint32_t qa[4], qb[4];
+    for (int jj = 0; jj < 2; ++jj) {
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            qa[w] = H.qh[4 * c + w] & 0x33333333u;         // bit pairs of groups 0 and 2
-            qb[w] = (H.qh[4 * c + w] >> 2) & 0x33333333u;  // of groups 1 and 3
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int c = 0; c < 2; ++c) {
             uint32_t code[4], o[8];
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
-                const uint32_t q = H.ql[(j & 1) * 8 + 4 * c + w], p = (j & 1) ? qb[w] : qa[w];
-                code[w] = j < 2 ? (q & m) | ((p << 4) & ~m) : ((q >> 4) & m) | (p & ~m);
+                const uint32_t q = H.ql[jj * 8 + 4 * c + w], p = H.qh[4 * c + w];
+                // the group's bit pairs, at bits 4-5 of each byte: group 2 K + jj has them at bits 4 K + 2 jj
+                const uint32_t two = (K == 0 ? (jj == 0 ? p << 4 : p << 2) : (jj == 0 ? p : p >> 2)) & 0x30303030u;
+                code[w] = ((K == 0 ? q : q >> 4) & m) | two;
             }
-            const int si = 2 * j + c;
+            const int si = 2 * (2 * K + jj) + c;
             const float sc = (float)(int)(int8_t)(H.sc[si >> 2] >> (8 * (si & 3)));
             pf_group(code, 0x64206420u, __float2half2_rn(H.d * sc), o);
-            tmem_st8(taddr + (uint32_t)(si * 8), o);
+            tmem_st8(taddr + (uint32_t)((2 * jj + c) * 8), o);
         }
     }
 }
@@ -401,12 +397,13 @@ __device__ __forceinline__ void pf_load8(uint32_t gb, uint32_t (&a)[36]) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) lds128(gb + 128u * H + 16u * i, a + 4 * i);
 }
-template <int H>
+// Stage K of the half: its blocks 2 K and 2 K + 1.
+template <int H, int K>
 __device__ __forceinline__ void pf_unpack8(const uint32_t (&a)[36], uint32_t taddr) {
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-        constexpr int base = 8 * H;
-        const int off = 34 * b + base, wi = off >> 2;  // the block's scale: low half of word wi (even b) or high half
+    for (int bb = 0; bb < 2; ++bb) {
+        const int b = 2 * K + bb;
+        const int off = 34 * b + 8 * H, wi = off >> 2;  // the block's scale: low half of word wi (even b) or high half
         const uint32_t dw = (b & 1) ? a[wi] >> 16 : a[wi];
         const __half2 ds2 = __float2half2_rn(__half2float(__ushort_as_half((unsigned short)dw)) * kPfWeightScale);
 #pragma unroll
@@ -418,7 +415,7 @@ __device__ __forceinline__ void pf_unpack8(const uint32_t (&a)[36], uint32_t tad
                 code[w] = ((b & 1) ? a[k + 1] : __byte_perm(a[k], a[k + 1], 0x5432)) ^ 0x80808080u;
             }
             pf_group(code, 0x64806480u, ds2, o);
-            tmem_st8(taddr + (uint32_t)((2 * b + g) * 8), o);
+            tmem_st8(taddr + (uint32_t)((2 * bb + g) * 8), o);
         }
     }
 }
@@ -427,32 +424,38 @@ __device__ __forceinline__ void pf_unpack8(const uint32_t (&a)[36], uint32_t tad
 struct PfCtl {
     uint64_t raw_full[kPfRawSlots];   // TMA bytes landed -> unpack warps
     uint64_t raw_empty[kPfRawSlots];  // unpack warps -> TMA thread
-    uint64_t a_full[kPfAStages];      // the eight unpack warps of a half -> MMA
-    uint64_t a_empty[kPfAStages];     // MMA (tcgen05.commit) -> unpack warps
-    uint64_t b_full[kPfMaxBStages];   // every loader lane (its copies landed) -> MMA
-    uint64_t b_empty[kPfMaxBStages];  // MMA (tcgen05.commit) -> B loaders
+    uint64_t full[kPfStages];         // the eight unpack warps of a half + every loader lane (its copies landed) -> MMA
+    uint64_t empty[kPfStages];        // MMA (tcgen05.commit) -> unpack warps and loaders
     uint64_t acc_full[2];             // MMA (tcgen05.commit) -> epilogue, by tile parity
     uint64_t acc_empty[2];            // epilogue -> MMA, by half of the accumulator columns
-    float* dst[2][kPfTileN];          // down, routed: result row of each token column, by tile parity
-    float factor[2][kPfTileN];        // and its routing weight
+    float* dst[kPfEpiTeams][2][kPfTileN];     // down, routed: result row of each token column, by tile parity
+    float factor[kPfEpiTeams][2][kPfTileN];   // and its routing weight
     uint32_t tmem_base;
     int abort_flag;
 };
 
-// The same verdict for all 128 epilogue threads: they meet in named barriers, so either all of them go on
-// or none does.
-__device__ __forceinline__ bool pf_epi_agree(bool ok) {
+// The same verdict for the 128 threads of an epilogue team: they meet in a named barrier, so either all of
+// them go on or none does.
+__device__ __forceinline__ bool pf_epi_agree(int team, bool ok) {
     uint32_t r;
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"((uint32_t)ok)
+        : "r"((uint32_t)ok), "r"(2 + team)
         : "memory");
     return r != 0;
 }
+__device__ __forceinline__ void pf_epi_sync(int team) { asm volatile("bar.sync %0, 128;" ::"r"(2 + team) : "memory"); }
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
 
-__host__ __device__ inline uint32_t pf_smem_bytes(int slot_bytes, int n_b) {
-    return 1024u + (uint32_t)n_b * kPfBStageBytes + 2u * kPfEpiBytes + (uint32_t)kPfRawSlots * (uint32_t)slot_bytes;
+__host__ __device__ inline uint32_t pf_smem_bytes(int slot_bytes) {
+    return 1024u + (uint32_t)kPfStages * kPfBStageBytes + 2u * kPfEpiTeams * kPfEpiBytes +
+           (uint32_t)kPfRawSlots * (uint32_t)slot_bytes;
 }
 
 // MODE_GATEUP (0): row tile 0 is gate rows 128 bx .. + 127, row tile 1 the same up rows.
@@ -468,10 +471,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
     const int n_shared = L.has_shared ? (valid + kPfTileN - 1) / kPfTileN : 0;
     const int n_tiles = (n_routed + n_shared) * L.row_units;
     const int n_spans = L.k / kSpanElems;
-    const int NB = L.n_b;
     uint8_t* bst = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    float* epi = (float*)(bst + (size_t)NB * kPfBStageBytes);
-    const uint32_t raw32 = smem_u32(epi) + 2u * kPfEpiBytes;
+    uint8_t* epi = bst + (size_t)kPfStages * kPfBStageBytes;
+    const uint32_t raw32 = smem_u32(epi) + 2u * kPfEpiTeams * kPfEpiBytes;
     volatile int* abortp = &ctl.abort_flag;
     const int G = gridDim.x;
 
@@ -481,17 +483,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
             mbar_init(&ctl.raw_full[i], 1);
             mbar_init(&ctl.raw_empty[i], kPfUnpackWarps);
         }
-        for (int i = 0; i < kPfAStages; ++i) {
-            mbar_init(&ctl.a_full[i], kPfUnpackWarps / 2);
-            mbar_init(&ctl.a_empty[i], 1);
-        }
-        for (int i = 0; i < NB; ++i) {
-            mbar_init(&ctl.b_full[i], kPfLoadWarps * 32);
-            mbar_init(&ctl.b_empty[i], 1);
+        for (int i = 0; i < kPfStages; ++i) {
+            mbar_init(&ctl.full[i], kPfUnpackWarps / 2 + kPfLoadWarps * 32);
+            mbar_init(&ctl.empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&ctl.acc_full[i], 1);
-            mbar_init(&ctl.acc_empty[i], 4);
+            mbar_init(&ctl.acc_empty[i], 4 * kPfEpiTeams);
         }
         fence_mbar_init();
     }
@@ -506,72 +504,79 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
 
     if (warp < kPfUnpackWarps) {
         // ------------------------------ unpack warps ------------------------------
-        // Warp 8 h + 4 rt + q: quadrant q (slots 32 q .. 32 q + 31) of row tile rt, half h of every span,
-        // which is also the A stage.
+        // Warp 8 h + 4 rt + q: quadrant q (slots 32 q .. 32 q + 31) of row tile rt, half h of every span, i.e.
+        // stages 2 h and 2 h + 1.
         const int q = warp & 3, rt = (warp >> 2) & 1, h = warp >> 3;
-        const uint32_t taddr = tmem_base + kPfColsA + (uint32_t)(h * 2 + rt) * 64u + ((uint32_t)(q * 32) << 16);
+        const uint32_t taddr = tmem_base + kPfColsA + (uint32_t)h * 128u + (uint32_t)rt * 32u + ((uint32_t)(q * 32) << 16);
         uint32_t n = 0;  // spans since the kernel started
         bool ok = true;
-        PfTile T{}, T1{};
-        if ((int)blockIdx.x < n_tiles) T = pf_tile(L, blockIdx.x, n_routed, valid);
         for (int t = blockIdx.x; t < n_tiles && ok; t += G) {
-            if (t + G < n_tiles) T1 = pf_tile(L, t + G, n_routed, valid);  // in flight during this tile
-            const int quant = T.shared ? QS : QR;
+            const int quant = t / L.row_units >= n_routed ? QS : QR;
             const int span_b = span_bytes_of(quant), box = (int)rows_box_bytes(quant);
             const int row_b = n_spans * span_b, R = pf_row_group((uint32_t)row_b);
-            const int cls = (32 * q + lane) / (kPfTileM / R);
+            const int x0 = (32 * q + lane) / (kPfTileM / R) * row_b;
+            const uint32_t row32 = raw32 + (uint32_t)((rt * kPfTileM + q * 32 + lane) * box);
             for (int s = 0; s < n_spans; ++s, ++n) {
                 const int slot = (int)(n & 1);
                 ok = warp_wait_pf(&ctl.raw_full[slot], (n >> 1) & 1, abortp, L.status);
                 if (!ok) break;
-                const int x = cls * row_b + s * span_b;
+                const int x = x0 + s * span_b;
                 const uint32_t delta = (uint32_t)(x - rows_box_start(x, R * row_b, box));
-                const uint32_t gb = raw32 + (uint32_t)(slot * L.slot_bytes + (rt * kPfTileM + q * 32 + lane) * box) + (delta & ~15u);
-                auto stage_free = [&]() -> bool {
+                const uint32_t gb = row32 + (uint32_t)(slot * L.slot_bytes) + (delta & ~15u);
+                auto stage_free = [&](int k) -> bool {
                     bool o = true;
-                    if (n >= 1) o = warp_wait_pf(&ctl.a_empty[h], (n - 1) & 1, abortp, L.status);
+                    if (n >= 1) o = warp_wait_pf(&ctl.empty[2 * h + k], (n - 1) & 1, abortp, L.status);
                     tc_fence_after();
                     return o;
+                };
+                auto stage_done = [&](int k) {
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive32(smem_u32(&ctl.full[2 * h + k]));
                 };
                 if (quant == QUANT_Q6K) {
                     PfHalf6 H;
                     pf_load6(gb, (delta & 15u) >> 1, h, H);
-                    ok = stage_free();
-                    if (!ok) break;
-                    pf_unpack6(H, taddr);
+                    if (!(ok = stage_free(0))) break;
+                    pf_unpack6<0>(H, taddr);
+                    stage_done(0);
+                    if (!(ok = stage_free(1))) break;
+                    pf_unpack6<1>(H, taddr + 64u);
+                    stage_done(1);
                 } else {
                     uint32_t a[36];
                     if (h == 0) {
                         pf_load8<0>(gb, a);
-                        ok = stage_free();
-                        if (!ok) break;
-                        pf_unpack8<0>(a, taddr);
+                        if (!(ok = stage_free(0))) break;
+                        pf_unpack8<0, 0>(a, taddr);
+                        stage_done(0);
+                        if (!(ok = stage_free(1))) break;
+                        pf_unpack8<0, 1>(a, taddr + 64u);
                     } else {
                         pf_load8<1>(gb, a);
-                        ok = stage_free();
-                        if (!ok) break;
-                        pf_unpack8<1>(a, taddr);
+                        if (!(ok = stage_free(0))) break;
+                        pf_unpack8<1, 0>(a, taddr);
+                        stage_done(0);
+                        if (!(ok = stage_free(1))) break;
+                        pf_unpack8<1, 1>(a, taddr + 64u);
                     }
+                    stage_done(1);
                 }
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive32(smem_u32(&ctl.a_full[h]));
-                    // Only here is it certain that the raw bytes have been read: an arrival right behind the
-                    // shared loads (whose results nothing had used yet) let the next span's copy overtake them.
-                    mbar_arrive32(smem_u32(&ctl.raw_empty[slot]));
-                }
+                // Only here is it certain that the raw bytes have been read: an arrival right behind the shared
+                // loads (whose results nothing had used yet) let the next span's copy overtake them.
+                if (lane == 0) mbar_arrive32(smem_u32(&ctl.raw_empty[slot]));
             }
-            T = T1;
         }
     } else if (warp < kPfWarpMma) {
         // ------------------------------- epilogue -------------------------------
-        // Thread (quad, lane) owns slot 32 quad + lane of both row tiles: tensor-memory lane = weight row,
-        // column = token.  Sixteen tokens at a time pass through shared memory as [token][slot]; then a warp
-        // takes four of the tokens and a lane four neighbouring output rows of each.
-        const int quad = warp & 3, etid = tid - 32 * kPfWarpEpi0, lslot = quad * 32 + lane;
+        // Thread (quad, lane) of a team owns slot 32 quad + lane: tensor-memory lane = weight row, column =
+        // token.  The outputs of sixteen tokens (gate/up, f16, two tokens to a word) or eight (down) pass through
+        // shared memory as [token][slot]; then a warp takes four or two of the tokens and a lane four neighbouring
+        // output rows of each.  Gate/up: the teams take sixteen tokens in turn; down: a row tile each.
+        const int team = (warp - kPfWarpEpi0) >> 2, quad = warp & 3, etid = quad * 32 + lane;
         const float inv = 1.0f / kPfWeightScale;
+        uint8_t* bufs = epi + team * 2 * kPfEpiBytes;
         uint32_t n = 0, nbuf = 0, half_sel = 0;
         for (int t = blockIdx.x; t < n_tiles; t += G, ++n) {
             const PfTile T = pf_tile(L, t, n_routed, valid);
@@ -591,11 +596,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                     f = __ldg(L.topk_weights + flat) * inv;  // a power of two: folded in exactly
                     p = result_row(L.partial, L.partial_rows, flat, L.rows);
                 }
-                ctl.dst[tp][etid] = p;
-                ctl.factor[tp][etid] = f;
+                ctl.dst[team][tp][etid] = p;
+                ctl.factor[team][tp][etid] = f;
             }
             bool ok = warp_wait_pf<true>(&ctl.acc_full[tp], (n >> 1) & 1, abortp, L.status);
-            ok = pf_epi_agree(ok);
+            ok = pf_epi_agree(team, ok);
             if (!ok) break;
             tc_fence_after();
             const uint32_t tq = tmem_base + half * 64u + ((uint32_t)(quad * 32) << 16);
@@ -608,74 +613,88 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                     if (two || half == 1) mbar_arrive32(smem_u32(&ctl.acc_empty[1]));
                 }
             };
-            constexpr int RTS = MODE == MODE_GATEUP ? 1 : 2;
+            // the four words of row [128] that hold output rows 4 lane .. 4 lane + 3 of the tile
+            auto quad_of = [&](const uint32_t* src) -> uint4 {
+                if (R == 1) return *(const uint4*)(src + 4 * lane);
+                if (R == 2) {
+                    const uint2 a = *(const uint2*)(src + 2 * lane), b = *(const uint2*)(src + 64 + 2 * lane);
+                    return make_uint4(a.x, b.x, a.y, b.y);
+                }
+                if (R == 4) return make_uint4(src[lane], src[32 + lane], src[64 + lane], src[96 + lane]);
+                const uint32_t* p = src + (lane & 1) * 64 + (lane >> 1);
+                return make_uint4(p[0], p[16], p[32], p[48]);
+            };
+            if (MODE == MODE_GATEUP) {
+                if (team >= steps) release();
 #pragma unroll 1
-            for (int rt = 0; rt < RTS; ++rt) {
-#pragma unroll 1
-                for (int st = 0; st < steps; ++st, ++nbuf) {
-                    float* buf = epi + (nbuf & 1) * (kPfEpiBytes / 4);
-                    uint32_t r[16];
-                    tmem_ld16(tq + (uint32_t)(rt * 128 + st * kPfEpiTokens), r);
-                    if (MODE == MODE_GATEUP) {
-                        uint32_t u[16];
-                        tmem_ld16(tq + (uint32_t)(128 + st * kPfEpiTokens), u);
-                        tmem_ld_wait16(r);
-                        tmem_ld_wait16(u);
-                        if (st == steps - 1) release();
+                for (int st = team; st < steps; st += kPfEpiTeams, ++nbuf) {
+                    uint32_t* buf = (uint32_t*)(bufs + (nbuf & 1) * kPfEpiBytes);
+                    uint32_t r[16], u[16];
+                    tmem_ld16(tq + (uint32_t)(st * kPfEpiTokens), r);
+                    tmem_ld16(tq + (uint32_t)(128 + st * kPfEpiTokens), u);
+                    tmem_ld_wait16(r);
+                    tmem_ld_wait16(u);
+                    if (st + kPfEpiTeams >= steps) release();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float gv = __uint_as_float(r[i]) * inv, uv = __uint_as_float(u[i]) * inv;
-                            buf[i * kPfTileM + lslot] = swiglu_fast(gv, uv);
-                        }
-                    } else {
-                        tmem_ld_wait16(r);
-                        if (rt == RTS - 1 && st == steps - 1) release();
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) buf[i * kPfTileM + lslot] = __uint_as_float(r[i]);
+                    for (int i = 0; i < 8; ++i) {
+                        const __half2 v = __floats2half2_rn(
+                            swiglu_fast(__uint_as_float(r[2 * i]) * inv, __uint_as_float(u[2 * i]) * inv),
+                            swiglu_fast(__uint_as_float(r[2 * i + 1]) * inv, __uint_as_float(u[2 * i + 1]) * inv));
+                        buf[i * kPfTileM + etid] = *(const uint32_t*)&v;
                     }
-                    asm volatile("bar.sync 2, 128;" ::: "memory");  // the four epilogue warps
+                    pf_epi_sync(team);
                     // (the other buffer is rewritten only after every warp has passed the next barrier)
-                    float4 w[4];
+                    __half* out = (T.shared ? L.inter_shared : L.inter_routed) +
+                                  (size_t)(T.first + st * kPfEpiTokens) * L.rows + T.bx * kPfTileM + 4 * lane;
+                    uint4 w[2];
+                    w[0] = quad_of(buf + (2 * quad) * kPfTileM);
+                    w[1] = quad_of(buf + (2 * quad + 1) * kPfTileM);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const float* src = buf + (quad * 4 + k) * kPfTileM;
-                        float4& v = w[k];
-                        if (R == 1) {
-                            v = *(const float4*)(src + 4 * lane);
-                        } else if (R == 2) {
-                            const float2 a = *(const float2*)(src + 2 * lane), b = *(const float2*)(src + 64 + 2 * lane);
-                            v = make_float4(a.x, b.x, a.y, b.y);
-                        } else if (R == 4) {
-                            v = make_float4(src[lane], src[32 + lane], src[64 + lane], src[96 + lane]);
-                        } else {
-                            const float* p = src + (lane & 1) * 64 + (lane >> 1);
-                            v = make_float4(p[0], p[16], p[32], p[48]);
-                        }
+                        const int tok = 4 * quad + k;
+                        if (st * kPfEpiTokens + tok >= T.ncols) break;
+                        const uint4 v = w[k >> 1];
+                        const uint32_t sel = (k & 1) ? 0x7632u : 0x5410u;  // this token's halves
+                        *(uint2*)(out + (size_t)tok * L.rows) =
+                            make_uint2(__byte_perm(v.x, v.y, sel), __byte_perm(v.z, v.w, sel));
                     }
+                }
+            } else {
+#pragma unroll 1
+                for (int st = 0; st < steps; ++st) {
+                    uint32_t r[16];
+                    tmem_ld16(tq + (uint32_t)(team * 128 + st * kPfEpiTokens), r);
+                    tmem_ld_wait16(r);
+                    if (st == steps - 1) release();
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const int tok = st * kPfEpiTokens + quad * 4 + k;
-                        if (tok >= T.ncols) break;
-                        float4 v = w[k];
-                        if (MODE == MODE_GATEUP) {
-                            const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
-                            __half* dst = (T.shared ? L.inter_shared : L.inter_routed) + (size_t)(T.first + tok) * L.rows +
-                                          T.bx * kPfTileM + 4 * lane;
-                            *(uint2*)dst = make_uint2(*(const uint32_t*)&h0, *(const uint32_t*)&h1);
-                        } else {
-                            const int col = T.bx * 2 * kPfTileM + rt * kPfTileM + 4 * lane;
+                    for (int e = 0; e < 2; ++e, ++nbuf) {
+                        uint32_t* buf = (uint32_t*)(bufs + (nbuf & 1) * kPfEpiBytes);
+                        const int tok0 = st * kPfEpiTokens + 8 * e;
+                        if (tok0 >= T.ncols) break;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) buf[i * kPfTileM + etid] = r[8 * e + i];
+                        pf_epi_sync(team);
+                        const int col = T.bx * 2 * kPfTileM + team * kPfTileM + 4 * lane;
+                        uint4 w[2];
+                        w[0] = quad_of(buf + (2 * quad) * kPfTileM);
+                        w[1] = quad_of(buf + (2 * quad + 1) * kPfTileM);
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const int tok = tok0 + 2 * quad + k;
+                            if (tok >= T.ncols) break;
+                            const float f = T.shared ? inv : ctl.factor[team][tp][tok];
+                            const float4 v = make_float4(f * __uint_as_float(w[k].x), f * __uint_as_float(w[k].y),
+                                                         f * __uint_as_float(w[k].z), f * __uint_as_float(w[k].w));
                             if (T.shared) {
-                                v = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
                                 const size_t o = (size_t)(T.first + tok) * L.rows + col;
                                 *(float4*)(L.shexp + o) = v;
                                 if (L.l_out) {
-                                    const float4 e = *(const float4*)(L.residual + o);
-                                    *(float4*)(L.l_out + o) = make_float4(v.x + e.x, v.y + e.y, v.z + e.z, v.w + e.w);
+                                    const float4 e4 = *(const float4*)(L.residual + o);
+                                    *(float4*)(L.l_out + o) = make_float4(v.x + e4.x, v.y + e4.y, v.z + e4.z, v.w + e4.w);
                                 }
                             } else {
-                                const float f = ctl.factor[tp][tok];
-                                float* p = ctl.dst[tp][tok];
-                                if (p) *(float4*)(p + col) = make_float4(f * v.x, f * v.y, f * v.z, f * v.w);
+                                float* p = ctl.dst[team][tp][tok];
+                                if (p) *(float4*)(p + col) = v;
                             }
                         }
                     }
@@ -684,69 +703,59 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
         }
     } else if (warp == kPfWarpMma) {
         // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
-            uint32_t n = 0, tn = 0, half_sel = 0, uses[2] = {0, 0};
-            int bs = 0;
-            uint32_t bph = 0;
-            bool ok = true;
-            PfTile T{}, T1{};
-            if ((int)blockIdx.x < n_tiles) T = pf_tile(L, blockIdx.x, n_routed, valid);
-            for (int t = blockIdx.x; t < n_tiles && ok; t += G, ++tn) {
-                if (t + G < n_tiles) T1 = pf_tile(L, t + G, n_routed, valid);
-                const uint32_t idesc = umma_idesc_f16(kPfTileM, (T.ncols + 15) & ~15);
-                // Accumulator columns: row tile rt owns columns 128 rt .. + 127; a tile of up to 64 tokens takes
-                // one half of them, alternately, a wider one both.
-                uint32_t half = 0;
-                const bool two = T.ncols > kPfTileN / 2;
-                if (!two) {
-                    half = half_sel;
-                    half_sel ^= 1u;
-                }
-                for (uint32_t r = 0; r < 2 && ok; ++r) {
-                    if (!two && r != half) continue;
-                    if (uses[r] >= 1) ok = stream_wait_pf(&ctl.acc_empty[r], (uses[r] - 1) & 1, abortp, L.status);
-                    ++uses[r];
-                }
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t d0 = tmem_base + half * 64u;
-                for (int s = 0; s < n_spans && ok; ++s, ++n) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {  // straight-line code for the whole span
-                        if (!stream_wait_pf(&ctl.a_full[h], n & 1, abortp, L.status)) {
-                            ok = false;
-                            break;
-                        }
-                        const uint32_t ta = tmem_base + kPfColsA + (uint32_t)h * 128u;
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            if (!stream_wait_pf(&ctl.b_full[bs], bph, abortp, L.status)) {
-                                ok = false;
-                                break;
-                            }
-                            tc_fence_after();
-                            if (MODE == MODE_GATEUP) fence_proxy_async_smem();  // rows that arrived by cp.async
-                            const uint64_t xdesc = umma_smem_desc(smem_u32(bst) + (uint32_t)bs * kPfBStageBytes);
-                            const uint32_t tc = ta + (uint32_t)c * 32u;
-#pragma unroll
-                            for (int rt = 0; rt < 2; ++rt)
-#pragma unroll
-                                for (int k4 = 0; k4 < 4; ++k4)  // 32 bytes per K16 step inside the swizzle row
-                                    umma_f16_ta(d0 + (uint32_t)rt * 128u, tc + (uint32_t)(rt * 64 + k4 * 8), xdesc + 2 * k4,
-                                                idesc, (s > 0 || h > 0 || c > 0 || k4 > 0) ? 1u : 0u);
-                            umma_commit(&ctl.b_empty[bs]);
-                            if (++bs == NB) {
-                                bs = 0;
-                                bph ^= 1u;
-                            }
-                        }
-                        if (!ok) break;
-                        umma_commit(&ctl.a_empty[h]);
-                    }
-                }
-                if (ok) umma_commit(&ctl.acc_full[tn & 1]);
-                T = T1;
+        // The whole warp walks the loop, so that addresses stay in uniform registers; one lane issues.
+        uint32_t n = 0, tn = 0, half_sel = 0, uses0 = 0, uses1 = 0;
+        bool ok = true;
+        PfTile T{}, T1{};
+        const uint64_t xdesc0 = umma_smem_desc(smem_u32(bst));
+        if ((int)blockIdx.x < n_tiles) T = pf_tile(L, blockIdx.x, n_routed, valid);
+        for (int t = blockIdx.x; t < n_tiles && ok; t += G, ++tn) {
+            if (t + G < n_tiles) T1 = pf_tile(L, t + G, n_routed, valid);
+            const uint32_t idesc = __shfl_sync(0xffffffffu, umma_idesc_f16(kPfTileM, (T.ncols + 15) & ~15), 0);
+            // Accumulator columns: row tile rt owns columns 128 rt .. + 127; a tile of up to 64 tokens takes
+            // one half of them, alternately, a wider one both.
+            uint32_t half = 0;
+            const bool two = T.ncols > kPfTileN / 2;
+            if (!two) {
+                half = half_sel;
+                half_sel ^= 1u;
             }
+            if (two || half == 0) {
+                if (uses0 >= 1) ok = warp_wait_pf(&ctl.acc_empty[0], (uses0 - 1) & 1, abortp, L.status);
+                ++uses0;
+            }
+            if (ok && (two || half == 1)) {
+                if (uses1 >= 1) ok = warp_wait_pf(&ctl.acc_empty[1], (uses1 - 1) & 1, abortp, L.status);
+                ++uses1;
+            }
+            if (!ok) break;
+            const uint32_t d0 = __shfl_sync(0xffffffffu, tmem_base + half * 64u, 0);
+            for (int s = 0; s < n_spans && ok; ++s, ++n) {
+#pragma unroll
+                for (int st = 0; st < kPfStages; ++st) {  // straight-line code for the whole span
+                    if (!warp_wait_pf(&ctl.full[st], n & 1, abortp, L.status)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    if (MODE == MODE_GATEUP) fence_proxy_async_smem();  // rows that arrived by cp.async
+                    if (elect_one()) {
+                        const uint64_t xdesc = xdesc0 + (uint64_t)(st * (kPfBStageBytes >> 4));
+                        const uint32_t ta = tmem_base + kPfColsA + (uint32_t)st * 64u;
+#pragma unroll
+                        for (int rt = 0; rt < 2; ++rt)
+#pragma unroll
+                            for (int k4 = 0; k4 < 4; ++k4)  // 32 bytes per K16 step inside the swizzle row
+                                umma_f16_ta(d0 + (uint32_t)rt * 128u, ta + (uint32_t)(rt * 32 + k4 * 8), xdesc + 2 * k4, idesc,
+                                            (s > 0 || st > 0 || k4 > 0) ? 1u : 0u);
+                        umma_commit(&ctl.empty[st]);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (ok && elect_one()) umma_commit(&ctl.acc_full[tn & 1]);
+            __syncwarp();
+            T = T1;
         }
     } else if (warp == kPfWarpRaw) {
         // ------------------------------ raw weight bytes ------------------------------
@@ -792,21 +801,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
         // are 8 i + 4 lw + lane / 8, i = 0 .. 15.
         const int lw = warp - kPfWarpLoad, piece = lane & 7, rlow = 4 * lw + (lane >> 3);
         const uint32_t b32 = smem_u32(bst), doff = b32 + swz_off(rlow, piece);
-        int bs = 0;
-        uint32_t bph = 0, issued = 0;
+        uint32_t issued = 0;  // stages since the kernel started
         bool ok = true;
         auto token_rows = [&](const PfTile& T, int (&xo)[16]) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int c = 8 * i + rlow;
                 xo[i] = !T.shared && c < T.ncols ? __ldg(L.sorted_token_ids + T.first + c) / L.top_k : -1;
-            }
-        };
-        auto advance = [&]() {
-            ++issued;
-            if (++bs == NB) {
-                bs = 0;
-                bph ^= 1u;
             }
         };
         // the tile record runs two tiles ahead of the work, the token rows one
@@ -823,34 +824,34 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
             if (MODE == MODE_GATEUP && !T.shared) {
                 const uint8_t* xb = (const uint8_t*)L.x_routed + piece * 16;
                 const size_t pitch = (size_t)L.k * 2;
-                for (int c = 0; c < L.k / kPfChunkK; ++c, xb += 2 * kPfChunkK) {
-                    if (issued >= (uint32_t)NB) {
-                        ok = warp_wait_pf(&ctl.b_empty[bs], bph ^ 1u, abortp, L.status);
+                for (int c = 0; c < L.k / kPfChunkK; ++c, xb += 2 * kPfChunkK, ++issued) {
+                    const uint32_t bs = issued % kPfStages, use = issued / kPfStages;
+                    if (use >= 1) {
+                        ok = warp_wait_pf(&ctl.empty[bs], (use - 1) & 1, abortp, L.status);
                         if (!ok) break;
                     }
-                    const uint32_t dst = doff + (uint32_t)bs * kPfBStageBytes;
+                    const uint32_t dst = doff + bs * kPfBStageBytes;
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
                         if (xr[i] >= 0) cp_async16(dst + i * 1024u, xb + (size_t)xr[i] * pitch, 16u);
-                    cp_async_arrive_noinc(&ctl.b_full[bs]);
-                    advance();
+                    cp_async_arrive_noinc(&ctl.full[bs]);
                 }
             } else {
                 const CUtensorMap* tm = T.shared ? &L.tm_x_s : &L.tm_x_r;
                 const int boxes = (T.ncols + kPfBoxTokens - 1) / kPfBoxTokens;
-                for (int c = 0; c < L.k / kPfChunkK; ++c) {
-                    if (issued >= (uint32_t)NB) {
-                        ok = warp_wait_pf(&ctl.b_empty[bs], bph ^ 1u, abortp, L.status);
+                for (int c = 0; c < L.k / kPfChunkK; ++c, ++issued) {
+                    const uint32_t bs = issued % kPfStages, use = issued / kPfStages;
+                    if (use >= 1) {
+                        ok = warp_wait_pf(&ctl.empty[bs], (use - 1) & 1, abortp, L.status);
                         if (!ok) break;
                     }
-                    uint64_t* full = &ctl.b_full[bs];
+                    uint64_t* full = &ctl.full[bs];
                     if (lw == 0 && lane == 0) mbar_expect_tx(full, (uint32_t)boxes * kPfBoxTokens * kPfChunkK * 2u);
                     else mbar_arrive32(smem_u32(full));
                     __syncwarp();
                     if (lw == 0 && lane < boxes)
-                        tma_load_box_2d32(b32 + (uint32_t)bs * kPfBStageBytes + (uint32_t)lane * (kPfBoxTokens * 128u), tm,
-                                          c * kPfChunkK, T.first + lane * kPfBoxTokens, full);
-                    advance();
+                        tma_load_box_2d32(b32 + bs * kPfBStageBytes + (uint32_t)lane * (kPfBoxTokens * 128u), tm, c * kPfChunkK,
+                                          T.first + lane * kPfBoxTokens, full);
                 }
             }
             T = T1;
@@ -861,15 +862,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        // after an abort: let the boxes in flight land before the CTA's shared memory is handed on
+        // After an abort: let the boxes in flight land before the CTA's shared memory is handed on.  (A stage's
+        // barrier may never complete when the unpack warps have left, so this waits for time, bounded.)
         if (!ok)
-            for (uint32_t back = 0; back < (uint32_t)NB && back < issued; ++back) {
-                if (--bs < 0) {
-                    bs = NB - 1;
-                    bph ^= 1u;
-                }
-                for (uint32_t it = 0; it < kWaitLimit; ++it)
-                    if (mbar_try_wait(&ctl.b_full[bs], bph)) break;
+            for (uint32_t back = 0; back < (uint32_t)kPfStages && back < issued; ++back) {
+                const uint32_t u = issued - 1 - back;
+                for (uint32_t it = 0; it < 1024u; ++it)
+                    if (mbar_try_wait(&ctl.full[u % kPfStages], (u / kPfStages) & 1)) break;
             }
     }
     // every thread of the CTA arrives here on every path, so tensor memory is always returned

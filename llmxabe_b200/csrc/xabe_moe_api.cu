@@ -479,14 +479,12 @@ int launch_prefill_t(xabe_moe* m, cudaStream_t st, const PrefillLaunch& L, uint3
 }
 template <int MODE>
 int launch_prefill(xabe_moe* m, cudaStream_t st, PrefillLaunch& L, int qr, int qs) {
-    // one CTA per SM; the B ring takes what the raw slots of the longer row format leave
+    // one CTA per SM
     int box = 0;
     if (L.has_routed) box = (int)rows_box_bytes(qr == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
     if (L.has_shared) box = std::max(box, (int)rows_box_bytes(qs == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0));
     L.slot_bytes = 2 * kPfTileM * box;
-    L.n_b = kPfMaxBStages;
-    while (L.n_b > 2 && pf_smem_bytes(L.slot_bytes, L.n_b) > 223u * 1024u) --L.n_b;
-    const uint32_t smem = pf_smem_bytes(L.slot_bytes, L.n_b);
+    const uint32_t smem = pf_smem_bytes(L.slot_bytes);
     if (qr == XABE_QUANT_Q6_K)
         return qs == XABE_QUANT_Q6_K ? launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q6K>(m, st, L, smem)
                                      : launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q8_0>(m, st, L, smem);
