@@ -159,6 +159,7 @@ struct xabe_moe {
     int* chunk_hist = nullptr;
     int* expert_offsets = nullptr;
     int* expert_counts = nullptr;
+    int* group_base = nullptr;  // [num_experts] column groups before each expert's
     int* work_items = nullptr;  // column groups, kWorkItemInts ints each
     int* n_work = nullptr;      // device scalar: routed column groups this step
     uint64_t work_capacity = 0;
@@ -935,15 +936,15 @@ int launch_route_and_dispatch(xabe_moe* m, cudaStream_t st, const float* logits)
     size_t hist_bytes = (size_t)(g.num_experts + 1) * sizeof(int);
     if ((uint64_t)g.max_tokens * g.experts_per_token <= (uint64_t)kSmallPairs) {
         // decode widths: one single-CTA launch
-        size_t smem = dispatch_small_smem((int)g.num_experts, 256);
+        const size_t smem = dispatch_small_smem((int)g.num_experts);
         const float* fused_logits = logits;
-        if (logits && g.max_tokens > 8) {  // more than one token per warp: route on many SMs first
+        if (logits && g.max_tokens > 8) {  // route on many SMs first
             CUDA_TRY(launch_pdl(m->pdl, k_route, dim3((g.max_tokens + 7) / 8), dim3(256), 0, st, logits,
                                 (const int*)m->valid_tokens, (int)g.num_experts, (int)g.experts_per_token,
                                 m->topk_ids, m->topk_weights));
             fused_logits = nullptr;
         }
-        CUDA_TRY(launch_pdl(m->pdl, k_route_dispatch_small, dim3(1), dim3(256), smem, st, fused_logits,
+        CUDA_TRY(launch_pdl(m->pdl, k_route_dispatch_small, dim3(1), dim3(kDispatchThreads), smem, st, fused_logits,
                             (const int*)m->valid_tokens, (int)g.num_experts, (int)g.experts_per_token,
                             (int)g.block_size, (int)m->sorted_capacity, (int)m->block_capacity, m->topk_ids,
                             m->topk_weights, m->sorted_token_ids, m->expert_ids, m->num_tokens_post_pad,
@@ -966,26 +967,24 @@ int launch_route_and_dispatch(xabe_moe* m, cudaStream_t st, const float* logits)
                                                       (int)m->block_capacity, m->chunk_hist,
                                                       m->sorted_token_ids, m->expert_ids);
     CUDA_TRY(cudaGetLastError());
+    // Only the work list of the kernels that will run: the regime must be chosen before this call.
+    const bool tc = prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate);
     int threads = ((int)g.num_experts + 31) / 32 * 32;
     k_align_scan<<<1, threads, 0, counted(st)>>>((int)g.num_experts, m->n_chunks, (int)g.block_size,
                                                  m->chunk_hist, m->expert_offsets, m->expert_counts,
-                                                 m->expert_ids, m->num_tokens_post_pad);
+                                                 m->expert_ids, m->num_tokens_post_pad, m->group_base,
+                                                 tc ? nullptr : m->n_work);
     CUDA_TRY(cudaGetLastError());
-    k_align_scatter<<<m->n_chunks, 32, hist_bytes, counted(st)>>>(m->topk_ids, m->valid_tokens,
-                                                        (int)g.experts_per_token, (int)g.num_experts,
-                                                        m->align_chunk, m->chunk_hist, m->expert_offsets,
-                                                        m->sorted_token_ids);
+    k_align_scatter<<<m->n_chunks, 32, hist_bytes, counted(st)>>>(
+        m->topk_ids, m->valid_tokens, (int)g.experts_per_token, (int)g.num_experts, m->align_chunk, m->chunk_hist,
+        m->expert_offsets, m->sorted_token_ids, m->expert_counts, m->group_base, m->topk_weights,
+        tc ? nullptr : m->work_items);
     CUDA_TRY(cudaGetLastError());
-    // Only the work list of the kernels that will run: the regime must be chosen before this call.
-    if (prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate)) {
+    if (tc) {
         k_build_prefill_items<<<1, threads, hist_bytes, counted(st)>>>((int)g.num_experts, m->expert_offsets,
                                                               m->expert_counts, m->pf_items, m->pf_n_items, kPfTileN);
-    } else {
-        k_build_work<<<1, threads, hist_bytes, counted(st)>>>((int)g.num_experts, m->expert_offsets, m->expert_counts,
-                                                     m->sorted_token_ids, m->topk_weights, m->work_items,
-                                                     m->n_work);
+        CUDA_TRY(cudaGetLastError());
     }
-    CUDA_TRY(cudaGetLastError());
     return XABE_OK;
 }
 
@@ -1059,7 +1058,7 @@ int launch_front(xabe_moe* m, cudaStream_t st, const float* x, const xabe_moe_la
     if (!with_routing) return launch_route_and_dispatch(m, st, m->logits);
     if (P.fused_dispatch) return rc;
     // wider handles: the tables from the routing the launch above stored (256 threads, one CTA)
-    CUDA_TRY(launch_pdl(m->pdl, k_route_dispatch_small, dim3(1), dim3(256), dispatch_small_smem((int)g.num_experts, 256),
+    CUDA_TRY(launch_pdl(m->pdl, k_route_dispatch_small, dim3(1), dim3(kDispatchThreads), dispatch_small_smem((int)g.num_experts),
                         st, (const float*)nullptr, (const int*)m->valid_tokens, (int)g.num_experts,
                         (int)g.experts_per_token, (int)g.block_size, (int)m->sorted_capacity, (int)m->block_capacity,
                         m->topk_ids, m->topk_weights, m->sorted_token_ids, m->expert_ids, m->num_tokens_post_pad,
@@ -1173,6 +1172,7 @@ int xabe_moe_create(const xabe_moe_geometry* geometry, int device, int scope, fl
         A(dev_alloc(&m->chunk_hist, (size_t)m->n_chunks * E));
         A(dev_alloc(&m->expert_offsets, E + 1));
         A(dev_alloc(&m->expert_counts, E + 1));
+        A(dev_alloc(&m->group_base, E + 1));
         A(dev_alloc(&m->front_tickets, T + 1));
         A(dev_alloc(&m->tail_done, (size_t)kTailMaxTokens * (H / 128 + 1)));
         A(dev_alloc(&m->ep_compact, E + 1));
@@ -1212,7 +1212,7 @@ void xabe_moe_destroy(xabe_moe* m) {
     if (!m) return;
     cudaSetDevice(m->device);
     void* dev[] = {m->valid_tokens, m->status, m->topk_ids, m->topk_weights, m->sorted_token_ids, m->expert_ids,
-                   m->num_tokens_post_pad, m->chunk_hist, m->expert_offsets, m->expert_counts, m->front_tickets, m->tail_done, m->ep_compact, m->ep_rank_start, m->ep_send_counts, m->work_items, m->n_work, m->pf_items,
+                   m->num_tokens_post_pad, m->chunk_hist, m->expert_offsets, m->expert_counts, m->group_base, m->front_tickets, m->tail_done, m->ep_compact, m->ep_rank_start, m->ep_send_counts, m->work_items, m->n_work, m->pf_items,
                    m->pf_n_items, m->normed, m->normed_h, m->logits,
                    m->inter_routed, m->inter_shared, m->dense_partial, m->partial, m->routed, m->shexp, m->gate, m->stage_in,
                    m->stage_ffn, m->stage_out};
