@@ -119,6 +119,19 @@ __device__ __forceinline__ float swiglu_fast(float g, float u) {
     return (q2 == q2 ? q2 : q) * u;  // (an infinite g has no remainder)
 }
 
+// (a0, a1) = (d0, d1) * s + (a0, a1): two independent fused multiply-adds in one instruction.
+__device__ __forceinline__ void fma2(float& a0, float& a1, float d0, float d1, uint64_t s) {
+    asm("{\n\t.reg .b64 x, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 z, {%0, %1};\n\tfma.rn.f32x2 z, x, %4, z;\n\t"
+        "mov.b64 {%0, %1}, z;\n\t}"
+        : "+f"(a0), "+f"(a1)
+        : "f"(d0), "f"(d1), "l"(s));
+}
+__device__ __forceinline__ uint64_t pack2(float v) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+
 // 32-bit word at a 2-byte-aligned shared-memory address.
 __device__ __forceinline__ uint32_t ld32_al2(const uint8_t* p) {
     uintptr_t a = (uintptr_t)p;

@@ -95,14 +95,20 @@ __device__ __forceinline__ void dense_half(const uint8_t* pa, const uint8_t* pb,
 #pragma unroll
         for (int q = 0; q < NG; ++q) b[q] = bnext[q];
         if (st < 7) fetch(st + 1);
+        const uint64_t sa = pack2(dsa), sb = pack2(dsb);
 #pragma unroll
         for (int q = 0; q < NG; ++q) {
             float d[4];
             mma_f16_16816(d, a, b[q].x, b[q].y);
-            acc[q][0] = fmaf(dsa, d[0], acc[q][0]);
-            acc[q][1] = fmaf(dsa, d[1], acc[q][1]);
-            acc[q][2] = fmaf(dsb, d[2], acc[q][2]);
-            acc[q][3] = fmaf(dsb, d[3], acc[q][3]);
+            if (NG == 1) {
+                acc[q][0] = fmaf(dsa, d[0], acc[q][0]);
+                acc[q][1] = fmaf(dsa, d[1], acc[q][1]);
+                acc[q][2] = fmaf(dsb, d[2], acc[q][2]);
+                acc[q][3] = fmaf(dsb, d[3], acc[q][3]);
+            } else {  // two groups and more repay the doubled scales
+                fma2(acc[q][0], acc[q][1], d[0], d[1], sa);
+                fma2(acc[q][2], acc[q][3], d[2], d[3], sb);
+            }
         }
     };
     if (QUANT == QUANT_Q6K) {
