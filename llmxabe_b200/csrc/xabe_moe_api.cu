@@ -164,6 +164,9 @@ struct xabe_moe {
     int* n_work = nullptr;      // device scalar: routed column groups this step
     uint64_t work_capacity = 0;
     int sm_count = 0;
+    cudaStream_t side = nullptr;     // the shared expert beside the dispatch (see forks_shared)
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    int grid_limit = 0;              // > 0: the streaming kernels' grid, while a launch shares the GPU
     int* pf_items = nullptr;    // token tiles for the tcgen05 prefill kernels
     int* pf_n_items = nullptr;
     uint64_t pf_capacity = 0;
@@ -323,12 +326,14 @@ StreamShape stream_shape(int mode, int rows, int k, int q_routed, int q_shared, 
     return sh;
 }
 
+inline unsigned stream_grid(const xabe_moe* m) { return (unsigned)(m->grid_limit > 0 ? m->grid_limit : m->sm_count); }
+
 template <int MODE, int QR, int QS>
 int launch_stream_t(xabe_moe* m, cudaStream_t st, const StreamLaunch& L, uint32_t smem) {
     auto kern = (MODE == MODE_DOWN && L.tail_done) ? k_expert_stream<MODE, QR, QS, MODE == MODE_DOWN>
                                                    : k_expert_stream<MODE, QR, QS, false>;
     CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-    CUDA_TRY(launch_pdl(m->pdl, kern, dim3(m->sm_count), dim3(kStreamThreads), smem, st, L));
+    CUDA_TRY(launch_pdl(m->pdl, kern, dim3(stream_grid(m)), dim3(kStreamThreads), smem, st, L));
     return XABE_OK;
 }
 
@@ -408,6 +413,9 @@ RowsShape rows_shape(const xabe_moe* m, int rows, int k, bool has_routed, int qr
         return true;
     };
     if (!fits(has_routed, qr, r_a, r_b) || !fits(has_shared, qs, s_a, s_b)) return sh;
+    // The shared expert alone has (tokens / 8) x (rows / 128) units.  Where that leaves half of the SMs without
+    // one, k_expert_stream's finer units are faster (19 tokens, 12 units: 16.4 -> 8 us; same sums).
+    if (!has_routed && (m->g.max_tokens + 7) / 8 * (uint32_t)(rows / kRowsUnitRows) * 2 < (uint32_t)m->sm_count) return sh;
     sh.stage_bytes = 2u * kRowsGroupRows * box;
     for (int S = kRowsMaxStages; S >= 3; --S) {
         RowsSmem R = rows_smem_layout(S, sh.stage_bytes, x_stride);
@@ -425,7 +433,7 @@ template <int QR, int QS>
 int launch_rows_t(xabe_moe* m, cudaStream_t st, const RowsLaunch& P, uint32_t smem) {
     auto kern = k_gateup_rows<QR, QS>;
     CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-    CUDA_TRY(launch_pdl(m->pdl, kern, dim3(m->sm_count), dim3(kStreamThreads), smem, st, P));
+    CUDA_TRY(launch_pdl(m->pdl, kern, dim3(stream_grid(m)), dim3(kStreamThreads), smem, st, P));
     return XABE_OK;
 }
 
@@ -537,6 +545,20 @@ struct DenseTail {
     float* l_out;
     bool done = false;
 };
+
+// Different formats for the routed experts and the shared expert (the shipped file: Q6_K and Q8_0) mean two
+// launches per projection (see run_experts).  The shared expert needs only the normalised rows, so on the
+// decode kernels it runs on a stream of the handle's own while the main stream routes and builds the
+// dispatch tables -- a chain of launches of a few CTAs.  Its grid leaves a quarter of the SMs to that chain: a
+// streaming CTA owns its SM.  Measured: 40 layers of 19 tokens 4913 -> 4210 us, one layer of 333 tokens
+// 371 -> 344 us, 64 tokens from host memory 240 -> 212 us; at one token the fork costs more than it hides (1380
+// -> 1476 us), so handles under 16 tokens keep the mixed launch.
+bool forks_shared(const xabe_moe* m, const xabe_moe_layer_weights* w) {
+    const auto& g = m->g;
+    return m->side && g.max_tokens >= 16 && !m->prof_on && !m->pdl && !m->force_tile_kernels &&
+           (w->gate_exps.quant != w->shared_gate.quant || w->down_exps.quant != w->shared_down.quant) &&
+           !prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate);
+}
 
 bool tail_applies(const xabe_moe* m, const xabe_moe_layer_weights* w) {
     const auto& g = m->g;
@@ -1190,6 +1212,11 @@ int xabe_moe_create(const xabe_moe_geometry* geometry, int device, int scope, fl
         A(dev_alloc(&m->routed, T * H));
         A(dev_alloc(&m->gate, T));
     }
+    if (scope == XABE_SCOPE_ROUTED) {
+        A(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
+        A(cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming));
+        A(cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming));
+    }
     if (g.max_tokens <= (uint32_t)kDrMaxTokens && H % 256 == 0) {
         // k_dense_rows<DOWN>: about as many units as SMs, by splitting the contraction as well
         const int row_blocks = (int)(H / 256), n_spans = (int)(I / 256);
@@ -1219,6 +1246,9 @@ void xabe_moe_destroy(xabe_moe* m) {
     for (void* p : dev)
         if (p) cudaFree(p);
     if (m->h_status) cudaFreeHost(m->h_status);
+    if (m->ev_fork) cudaEventDestroy(m->ev_fork);
+    if (m->ev_join) cudaEventDestroy(m->ev_join);
+    if (m->side) cudaStreamDestroy(m->side);
     if (m->prof_events) {
         for (int i = 0; i < kProfCalls * (XABE_STAGE_COUNT + 1); ++i) cudaEventDestroy(m->prof_events[i]);
         delete[] m->prof_events;
@@ -1597,6 +1627,25 @@ int xabe_moe_block_forward(xabe_moe* m, void* stream, const xabe_moe_layer_weigh
     const bool fused_front = front_applies(m, residual, w->router, &front_routes);
     const bool fused_tail = tail_applies(m, w) && ((uintptr_t)residual & 15) == 0 && ((uintptr_t)ffn_out & 15) == 0 &&
                             ((uintptr_t)l_out & 15) == 0;
+    MlpWeights r, s;
+    r.present = s.present = true;
+    r.gate = w->gate_exps;
+    r.up = w->up_exps;
+    r.down = w->down_exps;
+    s.gate = w->shared_gate;
+    s.up = w->shared_up;
+    s.down = w->shared_down;
+    const bool fork = !fused_tail && !fused_front && forks_shared(m, w);
+    auto fork_shared = [&]() -> int {  // the normalised rows are enqueued: the shared expert may follow them
+        CUDA_TRY(cudaEventRecord(m->ev_fork, st));
+        CUDA_TRY(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
+        m->grid_limit = m->sm_count * 3 / 4;
+        const int rcf = run_experts(m, m->side, MlpWeights{}, s, m->shexp);
+        m->grid_limit = 0;
+        CUDA_TRY(cudaEventRecord(m->ev_join, m->side));  // also after a failure: a capture must be joined
+        if (rcf) CUDA_TRY(cudaStreamWaitEvent(st, m->ev_join, 0));
+        return rcf;
+    };
     if (fused_front) {
         // one launch for norm, router, routing and dispatch: the stage profile books it under stage 0
         if ((rc = launch_front(m, st, residual, w, front_routes))) return rc;
@@ -1608,24 +1657,19 @@ int xabe_moe_block_forward(xabe_moe* m, void* stream, const xabe_moe_layer_weigh
         prof_mark(m, st, 1);
         if ((rc = launch_router(m, st, w->router, w->router_bias))) return rc;
         prof_mark(m, st, 2);
+        if (fork && (rc = fork_shared())) return rc;
         if ((rc = launch_route_and_dispatch(m, st, m->logits))) return rc;
     }
     prof_mark(m, st, 3);
-    MlpWeights r, s;
-    r.present = s.present = true;
-    r.gate = w->gate_exps;
-    r.up = w->up_exps;
-    r.down = w->down_exps;
-    s.gate = w->shared_gate;
-    s.up = w->shared_up;
-    s.down = w->shared_down;
     if (fused_tail) {
         // the down launch combines: routed, ffn_out and l_out are complete when it is
         const TailFusion tail{m->gate, residual, m->routed, ffn_out, l_out};
         if ((rc = run_experts(m, st, r, s, m->shexp, 4, &tail))) return rc;
         prof_mark(m, st, 5);
     } else {
-        if ((rc = run_experts(m, st, r, s, m->shexp, 4))) return rc;
+        rc = run_experts(m, st, r, fork ? MlpWeights{} : s, m->shexp, 4);
+        if (fork) CUDA_TRY(cudaStreamWaitEvent(st, m->ev_join, 0));
+        if (rc) return rc;
         prof_mark(m, st, 5);
         dim3 grid(g.max_tokens, g.max_tokens >= 512 ? 1u : (g.hidden + 255) / 256);
         CUDA_TRY(launch_pdl(m->pdl,
