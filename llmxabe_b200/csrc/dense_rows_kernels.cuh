@@ -70,9 +70,7 @@ __host__ __device__ inline uint32_t dense_rows_smem(int n_stages, int raw_pitch,
 }
 
 // Half a span (8 k16 steps) for fragment rows pa / pb against NG groups of eight token columns.
-// `xs`: this lane's column (row g of group 0) in the stage's activation slice.  (A run-time bound
-// on the groups that hold live rows was measured: the loop it leaves costs more than the skipped
-// groups save, 180 -> 240 us per layer at 64 tokens.)
+// `xs`: this lane's column (row g of group 0) in the stage's activation slice.
 template <int QUANT, bool MIS, int NG>
 __device__ __forceinline__ void dense_half(const uint8_t* pa, const uint8_t* pb, int h, const uint8_t* xs, int lane,
                                            float (&acc)[NG][4]) {
@@ -160,6 +158,99 @@ __device__ __forceinline__ void dense_half(const uint8_t* pa, const uint8_t* pb,
             a[2] = bytes23_to_h2(wa, bias128);
             a[3] = bytes23_to_h2(wb, bias128);
             step(a, dsa, dsb, st);
+        }
+    }
+}
+
+// A consumer warp's walk over its units with `NG` groups of eight token columns live.
+template <int MODE, int QUANT, int NG, typename Share>
+__device__ __forceinline__ void dense_consume(const DenseRowsLaunch& L, uint8_t* smem, uint64_t* full, uint64_t* empty,
+                                              uint32_t stage_bytes, int units, int valid, const Share& share,
+                                              volatile int* abortp) {
+    constexpr int span_b = QUANT == QUANT_Q6K ? 210 : 272;
+    constexpr int UNIT_ROWS = MODE == MODE_GATEUP ? 128 : 256;
+    const size_t row_bytes = (size_t)(L.k / kSpanElems) * span_b;
+    const int KS = MODE == MODE_GATEUP ? 1 : L.k_splits, S = L.n_stages;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cw = warp - kDrLoadWarps;
+    const int gi = cw / kStreamGroupWarps;  // which half of the unit's rows
+    const int w = cw % kStreamGroupWarps;   // warp within the group
+    const int g = lane >> 2, t = lane & 3;
+    int st = gi % S;
+    uint32_t use = (uint32_t)(gi / S);
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        const int rb = u / KS, ks = u - rb * KS;
+        int s0, s1;
+        share(ks, s0, s1);
+        const int first_row = rb * UNIT_ROWS + gi * (UNIT_ROWS / 2);
+        // fragment rows g and g + 8 of this warp: where they sit in a stage and in the matrices
+        int ra_slot, rb_slot;
+        uintptr_t ga, gb;  // global byte addresses of the two rows (only their low bits are used)
+        if (MODE == MODE_GATEUP) {
+            ra_slot = w * 8 + g;
+            rb_slot = 64 + w * 8 + g;
+            ga = (uintptr_t)(L.w_a + (size_t)(first_row + w * 8 + g) * row_bytes);
+            gb = (uintptr_t)(L.w_b + (size_t)(first_row + w * 8 + g) * row_bytes);
+        } else {
+            ra_slot = w * 16 + g;
+            rb_slot = w * 16 + g + 8;
+            ga = (uintptr_t)(L.w_a + (size_t)(first_row + ra_slot) * row_bytes);
+            gb = (uintptr_t)(L.w_a + (size_t)(first_row + rb_slot) * row_bytes);
+        }
+        float acc[NG][4];
+#pragma unroll
+        for (int q = 0; q < NG; ++q)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[q][i] = 0.f;
+        for (int s = s0; s < s1; ++s) {
+            if (!stream_wait(&full[st], use & 1, abortp, L.status)) return;
+            const uint8_t* slot = smem + (uint32_t)st * stage_bytes;
+            const uint8_t* pa = slot + (uint32_t)ra_slot * L.raw_pitch + (uint32_t)((ga + (size_t)s * span_b) & 15u);
+            const uint8_t* pb = slot + (uint32_t)rb_slot * L.raw_pitch + (uint32_t)((gb + (size_t)s * span_b) & 15u);
+            const uint8_t* xs = slot + (uint32_t)(kDrStageRows * L.raw_pitch) + (uint32_t)g * kDrXPitch;
+            // every row pitch is a multiple of four bytes (checked by the host), so the two rows and
+            // all lanes of the warp share one word alignment
+            if ((uintptr_t)pa & 2) {
+                dense_half<QUANT, true, NG>(pa, pb, 0, xs, lane, acc);
+                dense_half<QUANT, true, NG>(pa, pb, 1, xs, lane, acc);
+            } else {
+                dense_half<QUANT, false, NG>(pa, pb, 0, xs, lane, acc);
+                dense_half<QUANT, false, NG>(pa, pb, 1, xs, lane, acc);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[st]);  // the ring stage may be refilled
+            st += kStreamGroups;
+            if (st >= S) {
+                st -= S;
+                ++use;
+            }
+        }
+        if (MODE == MODE_GATEUP) {
+            // SwiGLU of this warp's eight rows: acc[.][0..1] gate, acc[.][2..3] up, columns 2t and 2t + 1
+            const int row = first_row + w * 8 + g;
+#pragma unroll
+            for (int q = 0; q < NG; ++q)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int tok = q * 8 + 2 * t + i;
+                    if (tok < valid) {
+                        const float gv = acc[q][i], uv = acc[q][2 + i];
+                        L.inter[(size_t)tok * L.rows + row] = __float2half_rn(__fdiv_rn(gv, 1.0f + expf(-gv)) * uv);
+                    }
+                }
+        } else {
+            const int row_lo = first_row + ra_slot, row_hi = first_row + rb_slot;
+            float* dst = L.out + (size_t)ks * L.max_tokens * L.rows;
+#pragma unroll
+            for (int q = 0; q < NG; ++q)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int tok = q * 8 + 2 * t + i;
+                    if (tok < valid) {
+                        dst[(size_t)tok * L.rows + row_lo] = acc[q][i];
+                        dst[(size_t)tok * L.rows + row_hi] = acc[q][2 + i];
+                    }
+                }
         }
     }
 }
@@ -262,87 +353,21 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
     }
 
     // ---------------------------------- consumers ----------------------------------
-    const int cw = warp - kDrLoadWarps;
-    const int gi = cw / kStreamGroupWarps;  // which half of the unit's rows
-    const int w = cw % kStreamGroupWarps;   // warp within the group
-    const int g = lane >> 2, t = lane & 3;
-    int st = gi % S;
-    uint32_t use = (uint32_t)(gi / S);
-    for (int u = blockIdx.x; u < units; u += gridDim.x) {
-        const int rb = u / KS, ks = u - rb * KS;
-        int s0, s1;
-        share(ks, s0, s1);
-        const int first_row = rb * UNIT_ROWS + gi * (UNIT_ROWS / 2);
-        // fragment rows g and g + 8 of this warp: where they sit in a stage and in the matrices
-        int ra_slot, rb_slot;
-        uintptr_t ga, gb;  // global byte addresses of the two rows (only their low bits are used)
-        if (MODE == MODE_GATEUP) {
-            ra_slot = w * 8 + g;
-            rb_slot = 64 + w * 8 + g;
-            ga = (uintptr_t)(L.w_a + (size_t)(first_row + w * 8 + g) * row_bytes);
-            gb = (uintptr_t)(L.w_b + (size_t)(first_row + w * 8 + g) * row_bytes);
-        } else {
-            ra_slot = w * 16 + g;
-            rb_slot = w * 16 + g + 8;
-            ga = (uintptr_t)(L.w_a + (size_t)(first_row + ra_slot) * row_bytes);
-            gb = (uintptr_t)(L.w_a + (size_t)(first_row + rb_slot) * row_bytes);
-        }
-        float acc[NG][4];
-#pragma unroll
-        for (int q = 0; q < NG; ++q)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[q][i] = 0.f;
-        for (int s = s0; s < s1; ++s) {
-            if (!stream_wait(&full[st], use & 1, abortp, L.status)) return;
-            const uint8_t* slot = smem + (uint32_t)st * stage_bytes;
-            const uint8_t* pa = slot + (uint32_t)ra_slot * L.raw_pitch + (uint32_t)((ga + (size_t)s * span_b) & 15u);
-            const uint8_t* pb = slot + (uint32_t)rb_slot * L.raw_pitch + (uint32_t)((gb + (size_t)s * span_b) & 15u);
-            const uint8_t* xs = slot + (uint32_t)(kDrStageRows * L.raw_pitch) + (uint32_t)g * kDrXPitch;
-            // every row pitch is a multiple of four bytes (checked by the host), so the two rows and
-            // all lanes of the warp share one word alignment
-            if ((uintptr_t)pa & 2) {
-                dense_half<QUANT, true, NG>(pa, pb, 0, xs, lane, acc);
-                dense_half<QUANT, true, NG>(pa, pb, 1, xs, lane, acc);
-            } else {
-                dense_half<QUANT, false, NG>(pa, pb, 0, xs, lane, acc);
-                dense_half<QUANT, false, NG>(pa, pb, 1, xs, lane, acc);
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[st]);  // the ring stage may be refilled
-            st += kStreamGroups;
-            if (st >= S) {
-                st -= S;
-                ++use;
-            }
-        }
-        if (MODE == MODE_GATEUP) {
-            // SwiGLU of this warp's eight rows: acc[.][0..1] gate, acc[.][2..3] up, columns 2t and 2t + 1
-            const int row = first_row + w * 8 + g;
-#pragma unroll
-            for (int q = 0; q < NG; ++q)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int tok = q * 8 + 2 * t + i;
-                    if (tok < valid) {
-                        const float gv = acc[q][i], uv = acc[q][2 + i];
-                        L.inter[(size_t)tok * L.rows + row] = __float2half_rn(__fdiv_rn(gv, 1.0f + expf(-gv)) * uv);
-                    }
-                }
-        } else {
-            const int row_lo = first_row + ra_slot, row_hi = first_row + rb_slot;
-            float* dst = L.out + (size_t)ks * L.max_tokens * L.rows;
-#pragma unroll
-            for (int q = 0; q < NG; ++q)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int tok = q * 8 + 2 * t + i;
-                    if (tok < valid) {
-                        dst[(size_t)tok * L.rows + row_lo] = acc[q][i];
-                        dst[(size_t)tok * L.rows + row_hi] = acc[q][2 + i];
-                    }
-                }
-        }
-    }
+    // As many groups as hold live tokens: a handle of 64 with 43 live ones runs the code for six groups, not for
+    // eight (164 -> 149 us per layer).  The code is chosen once per launch; a bound inside the loops cost more
+    // than it saved.
+    const int ng = (valid + 7) >> 3;
+    auto go = [&](auto N) {
+        dense_consume<MODE, QUANT, decltype(N)::value>(L, smem, full, empty, stage_bytes, units, valid, share, abortp);
+    };
+    if (NG >= 8 && ng > 7) go(std::integral_constant<int, 8>{});
+    else if (NG >= 8 && ng == 7) go(std::integral_constant<int, 7>{});
+    else if (NG >= 8 && ng == 6) go(std::integral_constant<int, 6>{});
+    else if (NG >= 8 && ng == 5) go(std::integral_constant<int, 5>{});
+    else if (NG >= 4 && ng == 4) go(std::integral_constant<int, 4>{});
+    else if (NG >= 4 && ng == 3) go(std::integral_constant<int, 3>{});
+    else if (NG >= 2 && ng == 2) go(std::integral_constant<int, 2>{});
+    else go(std::integral_constant<int, 1>{});
 }
 
 // out[t][j] = sum over ascending ks of partial[ks][t][j] for the live rows (MODE_DOWN with several
