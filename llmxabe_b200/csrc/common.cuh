@@ -126,10 +126,17 @@ __device__ __forceinline__ void fma2(float& a0, float& a1, float d0, float d1, u
         : "+f"(a0), "+f"(a1)
         : "f"(d0), "f"(d1), "l"(s));
 }
-__device__ __forceinline__ uint64_t pack2(float v) {
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
     uint64_t r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
     return r;
+}
+__device__ __forceinline__ uint64_t pack2(float v) { return pack2(v, v); }
+// The same with both factors packed.
+__device__ __forceinline__ void fma2(float& a0, float& a1, uint64_t x, uint64_t s) {
+    asm("{\n\t.reg .b64 z;\n\tmov.b64 z, {%0, %1};\n\tfma.rn.f32x2 z, %2, %3, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "+f"(a0), "+f"(a1)
+        : "l"(x), "l"(s));
 }
 
 // 32-bit word at a 2-byte-aligned shared-memory address.

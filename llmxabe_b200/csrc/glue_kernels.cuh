@@ -394,22 +394,37 @@ __global__ void __launch_bounds__(256, 1) k_router_logits_wide(const float* __re
 // is one lane group of every output, so the 32 trees of a token pair run inside the
 // warp (warp_trees32: no shared memory, no barrier); only the eight group totals
 // per output cross warps, through shared memory and one block barrier per ring stage.
-// grid: (E / 16, token shares); block 256;
-// dynamic shared memory: router_regw_smem(hidden).
+// grid: (E / (NE * PARTS), token shares); block 256 * PARTS;
+// dynamic shared memory: router_regw_smem(hidden, NE, PARTS).
 // ---------------------------------------------------------------------------
-constexpr int kRrOutputs = 32;                      // outputs per accumulator set: NE experts x 32 / NE tokens
-constexpr int kRrStageTokens = 4;                   // token rows per ring stage
-__host__ __device__ constexpr int rr_stages(int ne) { return ne == 16 ? 4 : 3; }
-
-__host__ __device__ inline size_t router_regw_smem(int hidden, int ne) {
-    return (size_t)rr_stages(ne) * kRrStageTokens * hidden * 4 + (size_t)2 * (kRrStageTokens * ne / 32) * kRrOutputs * 8 * 4;
+// warp_trees32 for accumulators in swizzled slots: slot s of lane l is output s ^ l.  What a lane keeps at a level
+// is then its lower slots and what it hands over its upper ones, whichever lane it is, so a level needs no
+// selection: the partner's slot s + off is this lane's output of slot s.  The sums are warp_trees32's.
+__device__ __forceinline__ float warp_trees32_swizzled(float (&acc)[32]) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int s = 0; s < off; ++s) acc[s] += __shfl_xor_sync(0xffffffffu, acc[s + off], off);
+    return acc[0];
 }
 
-// NE: expert rows per CTA held in registers.  16: one CTA per SM, two tokens per accumulator set.
-// 8: two CTAs per SM (half the weight registers), four tokens per set, a three-stage ring; twice as
-// many CTAs read each token row.
-template <int NI, int NE>
-__global__ void __launch_bounds__(256, NE == 16 ? 1 : 2) k_router_logits_regw(const float* __restrict__ w,
+constexpr int kRrOutputs = 32;                      // outputs per accumulator set: NE experts x 32 / NE tokens
+constexpr int kRrStageTokens = 8;                   // token rows per ring stage
+constexpr int kRrStages = 3;
+
+__host__ __device__ inline size_t router_regw_smem(int hidden, int ne, int parts) {
+    return (size_t)kRrStages * kRrStageTokens * hidden * 4 +
+           (size_t)parts * 2 * (kRrStageTokens * ne / 32) * kRrOutputs * 8 * 4;
+}
+
+// NE: expert rows a thread holds in registers; PARTS sets of 256 threads share the token ring of a CTA.
+// 8 rows and two sets (16 experts per CTA, four tokens per accumulator set) is the default.  What bounds it is
+// instruction issue: of a set's 370 instructions per thread 256 are the multiply-adds.  Measured at 16384 / 2048
+// tokens: one set per CTA, two CTAs per SM, trees with selections 591 / 79 us; two sets on one ring, eight
+// tokens per barrier, swizzled trees 512 / 76 us.  Paired multiply-adds (fma.rn.f32x2) are no faster, all of
+// them or half (579, 541 us): they save issue slots and lose them in the pipe.
+template <int NI, int NE, int PARTS>
+__global__ void __launch_bounds__(256 * PARTS, 1) k_router_logits_regw(const float* __restrict__ w,
                                                                const float* __restrict__ x,
                                                                const int* __restrict__ valid_tokens,
                                                                int num_experts, const float* __restrict__ bias,
@@ -419,13 +434,13 @@ __global__ void __launch_bounds__(256, NE == 16 ? 1 : 2) k_router_logits_regw(co
     pdl_wait();
     constexpr int hidden = NI * 256;
     constexpr int kRrTokens = kRrOutputs / NE;  // tokens per accumulator set
-    constexpr int kRrStages = rr_stages(NE);
     extern __shared__ __align__(128) float rr_smem[];
     float* xs = rr_smem;                                             // [stages][4][hidden]
-    float* group_tot = xs + kRrStages * kRrStageTokens * hidden;     // [2 stages][sets per stage][32][8]
+    constexpr int kPairs = kRrStageTokens / kRrTokens;  // accumulator sets per ring stage
+    const int part = threadIdx.x >> 8, tid = threadIdx.x & 255;
+    float* group_tot = xs + kRrStages * kRrStageTokens * hidden + part * (2 * kPairs * kRrOutputs * 8);  // [2 stages][sets][32][8]
     __shared__ __align__(8) uint64_t full[kRrStages];
-    const int tid = threadIdx.x;
-    const int e0 = blockIdx.x * NE;
+    const int e0 = (blockIdx.x * PARTS + part) * NE;
     const int live = *valid_tokens;
     // this CTA's tokens: a contiguous range, a whole number of stages except at the end of the batch
     const int stages_total = (live + kRrStageTokens - 1) / kRrStageTokens;
@@ -441,19 +456,19 @@ __global__ void __launch_bounds__(256, NE == 16 ? 1 : 2) k_router_logits_regw(co
                      &full[k % kRrStages]);
     };
     const int n_stages = stage1 - stage0;
-    if (tid == 0) {
+    if (threadIdx.x == 0) {
         for (int i = 0; i < kRrStages; ++i) mbar_init(&full[i], 1);
         fence_mbar_init();
         for (int k = 0; k < min(kRrStages, n_stages); ++k) issue(k);
     }
+    const int se = tid & (NE - 1), su = (tid & 31) / NE;  // this lane's slot swizzle (warp_trees32_swizzled)
     float wr[NE][NI];
 #pragma unroll
     for (int e = 0; e < NE; ++e)
 #pragma unroll
-        for (int i = 0; i < NI; ++i) wr[e][i] = __ldg(w + (size_t)(e0 + e) * hidden + i * 256 + tid);
+        for (int i = 0; i < NI; ++i) wr[e][i] = __ldg(w + (size_t)(e0 + (e ^ se)) * hidden + i * 256 + tid);
     __syncthreads();  // the barriers are initialised
     if (!__syncthreads_and(mbar_wait_bounded(&full[0], 0u, status))) return;
-    constexpr int kPairs = kRrStageTokens / kRrTokens;  // token pairs per ring stage
     for (int k = 0; k < n_stages; ++k) {
         const int slot = k % kRrStages;
         const float* xk = xs + (size_t)slot * kRrStageTokens * hidden;
@@ -464,23 +479,21 @@ __global__ void __launch_bounds__(256, NE == 16 ? 1 : 2) k_router_logits_regw(co
 #pragma unroll
         for (int p = 0; p < kPairs; ++p) {
             if (t_stage + p * kRrTokens >= live) break;  // uniform: the batch ended inside this stage
-            float acc[kRrOutputs];  // output o = e * tokens + u
-#pragma unroll
-            for (int o = 0; o < kRrOutputs; ++o) acc[o] = 0.0f;
+            float acc[kRrOutputs];  // slot u * NE + e: output (u ^ su) * NE + (e ^ se)
             // a row past the live tokens was not copied: its sums are formed from stale bytes and never stored
 #pragma unroll
             for (int i = 0; i < NI; ++i) {
                 float xv[kRrTokens];
 #pragma unroll
-                for (int u = 0; u < kRrTokens; ++u) xv[u] = xk[(p * kRrTokens + u) * hidden + i * 256 + tid];
+                for (int u = 0; u < kRrTokens; ++u) xv[u] = xk[(p * kRrTokens + (u ^ su)) * hidden + i * 256 + tid];
 #pragma unroll
-                for (int e = 0; e < NE; ++e)
+                for (int u = 0; u < kRrTokens; ++u)
 #pragma unroll
-                    for (int u = 0; u < kRrTokens; ++u)
-                        acc[e * kRrTokens + u] = fmaf(wr[e][i], xv[u], acc[e * kRrTokens + u]);
+                    for (int e = 0; e < NE; ++e)
+                        acc[u * NE + e] = fmaf(wr[e][i], xv[u], i == 0 ? 0.0f : acc[u * NE + e]);
             }
             // this warp is lane group tid / 32 of every output: its 32 trees, then lane o's total of output o
-            const float tot = warp_trees32(acc, tid & 31);
+            const float tot = warp_trees32_swizzled(acc);
             tot_stage[p * kRrOutputs * 8 + (tid & 31) * 8 + (tid >> 5)] = tot;
         }
         // One block barrier per stage: it publishes the group totals, tells thread 0 that every thread has
@@ -490,7 +503,7 @@ __global__ void __launch_bounds__(256, NE == 16 ? 1 : 2) k_router_logits_regw(co
         if (k + 1 < n_stages)
             ok = mbar_wait_bounded(&full[(k + 1) % kRrStages], (uint32_t)((k + 1) / kRrStages) & 1u, status);
         if (!__syncthreads_and(ok)) return;
-        if (tid == 0 && k + kRrStages < n_stages) issue(k + kRrStages);
+        if (threadIdx.x == 0 && k + kRrStages < n_stages) issue(k + kRrStages);
         // the eight group totals of an output, ascending, from +0; the pairs of a stage go to different warps
 #pragma unroll
         for (int p = 0; p < kPairs; ++p) {
@@ -501,7 +514,7 @@ __global__ void __launch_bounds__(256, NE == 16 ? 1 : 2) k_router_logits_regw(co
                 float total = 0.0f;
 #pragma unroll
                 for (int g = 0; g < 8; ++g) total += totb[o * 8 + g];
-                const int e = e0 + o / kRrTokens, t = t_stage + p * kRrTokens + o % kRrTokens;
+                const int e = e0 + o % NE, t = t_stage + p * kRrTokens + o / NE;
                 if (t < live && e < num_experts)
                     logits[(size_t)t * num_experts + e] = bias ? __fadd_rn(total, bias[e]) : total;
             }

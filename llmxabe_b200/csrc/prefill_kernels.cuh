@@ -74,7 +74,7 @@ constexpr int kPfStages = 4;        // one span: 64 contraction elements of both
 constexpr int kPfRawSlots = 2;      // one span of both row tiles each
 constexpr int kPfBoxTokens = 32;    // token rows of one box where they lie one after the other
 constexpr int kPfEpiTokens = 16;    // tokens an epilogue team reads at a time
-constexpr int kPfEpiBytes = 4096;   // what it turns around at a time; two buffers per team
+constexpr int kPfEpiBytes = 8192;   // what it turns around at a time (gate/up: half of it); one or two per team
 constexpr uint32_t kPfColsA = 256;  // tensor-memory column of the first A stage (accumulators below it)
 constexpr float kPfWeightScale = 256.0f;
 constexpr int kPfItemInts = 4;  // expert, first slot (or first token), columns, pad
@@ -111,6 +111,7 @@ struct PrefillLaunch {
     float* l_out;
     int* status;
     int row_units;   // tiles along the weight rows: gate/up rows / 128, down rows / 256
+    int epi_bufs;    // epilogue buffers per team: two where they fit beside the raw slots
     int slot_bytes;  // raw slot: 256 * the larger row pitch of the formats in this launch
 };
 
@@ -453,8 +454,8 @@ __device__ __forceinline__ bool elect_one() {
     return r != 0;
 }
 
-__host__ __device__ inline uint32_t pf_smem_bytes(int slot_bytes) {
-    return 1024u + (uint32_t)kPfStages * kPfBStageBytes + 2u * kPfEpiTeams * kPfEpiBytes +
+__host__ __device__ inline uint32_t pf_smem_bytes(int slot_bytes, int epi_bufs) {
+    return 1024u + (uint32_t)kPfStages * kPfBStageBytes + (uint32_t)(epi_bufs * kPfEpiTeams * kPfEpiBytes) +
            (uint32_t)kPfRawSlots * (uint32_t)slot_bytes;
 }
 
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
     const int n_spans = L.k / kSpanElems;
     uint8_t* bst = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* epi = bst + (size_t)kPfStages * kPfBStageBytes;
-    const uint32_t raw32 = smem_u32(epi) + 2u * kPfEpiTeams * kPfEpiBytes;
+    const uint32_t raw32 = smem_u32(epi) + (uint32_t)(L.epi_bufs * kPfEpiTeams * kPfEpiBytes);
     volatile int* abortp = &ctl.abort_flag;
     const int G = gridDim.x;
 
@@ -571,12 +572,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
     } else if (warp < kPfWarpMma) {
         // ------------------------------- epilogue -------------------------------
         // Thread (quad, lane) of a team owns slot 32 quad + lane: tensor-memory lane = weight row, column =
-        // token.  The outputs of sixteen tokens (gate/up, f16, two tokens to a word) or eight (down) pass through
-        // shared memory as [token][slot]; then a warp takes four or two of the tokens and a lane four neighbouring
-        // output rows of each.  Gate/up: the teams take sixteen tokens in turn; down: a row tile each.
+        // token.  The outputs of sixteen tokens (gate/up: f16, two tokens to a word) pass through shared memory as
+        // [token][slot]; then a warp takes four of the tokens and a lane four neighbouring output rows of each.
+        // Gate/up: the teams take sixteen tokens in turn; down: a row tile each.  The down projection has two
+        // spans of products per 256 x 128 outputs, so there the epilogue's latency is the launch:
+        // the next accumulators are fetched, and the rows' addresses read, under the barrier.  Eight tokens per
+        // barrier with everything behind it took 17 200 clocks a tile (561 us at 16384 tokens).
         const int team = (warp - kPfWarpEpi0) >> 2, quad = warp & 3, etid = quad * 32 + lane;
         const float inv = 1.0f / kPfWeightScale;
-        uint8_t* bufs = epi + team * 2 * kPfEpiBytes;
+        uint8_t* bufs = epi + team * L.epi_bufs * kPfEpiBytes;
         uint32_t n = 0, nbuf = 0, half_sel = 0;
         for (int t = blockIdx.x; t < n_tiles; t += G, ++n) {
             const PfTile T = pf_tile(L, t, n_routed, valid);
@@ -628,7 +632,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                 if (team >= steps) release();
 #pragma unroll 1
                 for (int st = team; st < steps; st += kPfEpiTeams, ++nbuf) {
-                    uint32_t* buf = (uint32_t*)(bufs + (nbuf & 1) * kPfEpiBytes);
+                    uint32_t* buf = (uint32_t*)(bufs + (nbuf & 1) * (kPfEpiBytes / 2));
                     uint32_t r[16], u[16];
                     tmem_ld16(tq + (uint32_t)(st * kPfEpiTokens), r);
                     tmem_ld16(tq + (uint32_t)(128 + st * kPfEpiTokens), u);
@@ -660,42 +664,49 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
                     }
                 }
             } else {
+                const int col = T.bx * 2 * kPfTileM + team * kPfTileM + 4 * lane;
+                const uint32_t tr = tq + (uint32_t)(team * 128);
+                uint32_t r[16];
+                tmem_ld16(tr, r);
 #pragma unroll 1
-                for (int st = 0; st < steps; ++st) {
-                    uint32_t r[16];
-                    tmem_ld16(tq + (uint32_t)(team * 128 + st * kPfEpiTokens), r);
+                for (int st = 0; st < steps; ++st, ++nbuf) {
+                    uint32_t* buf = (uint32_t*)(bufs + (nbuf & (uint32_t)(L.epi_bufs - 1)) * kPfEpiBytes);
                     tmem_ld_wait16(r);
                     if (st == steps - 1) release();
+                    // one buffer: every warp has read the step before (the first step: before pf_epi_agree); two:
+                    // a buffer is rewritten only after every warp has passed the barrier between
+                    if (L.epi_bufs == 1 && st > 0) pf_epi_sync(team);
 #pragma unroll
-                    for (int e = 0; e < 2; ++e, ++nbuf) {
-                        uint32_t* buf = (uint32_t*)(bufs + (nbuf & 1) * kPfEpiBytes);
-                        const int tok0 = st * kPfEpiTokens + 8 * e;
-                        if (tok0 >= T.ncols) break;
+                    for (int i = 0; i < 16; ++i) buf[i * kPfTileM + etid] = r[i];
+                    if (st < steps - 1) tmem_ld16(tr + (uint32_t)((st + 1) * kPfEpiTokens), r);
+                    float* p[4];
+                    float f[4];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) buf[i * kPfTileM + etid] = r[8 * e + i];
-                        pf_epi_sync(team);
-                        const int col = T.bx * 2 * kPfTileM + team * kPfTileM + 4 * lane;
-                        uint4 w[2];
-                        w[0] = quad_of(buf + (2 * quad) * kPfTileM);
-                        w[1] = quad_of(buf + (2 * quad + 1) * kPfTileM);
+                    for (int k = 0; k < 4; ++k) {
+                        const int tok = st * kPfEpiTokens + 4 * quad + k;
+                        const bool live = tok < T.ncols;
+                        if (T.shared) {
+                            p[k] = live ? L.shexp + (size_t)(T.first + tok) * L.rows : nullptr;
+                            f[k] = inv;
+                        } else {
+                            p[k] = live ? ctl.dst[team][tp][tok] : nullptr;
+                            f[k] = live ? ctl.factor[team][tp][tok] : 0.f;
+                        }
+                    }
+                    pf_epi_sync(team);
+                    uint4 w[4];
 #pragma unroll
-                        for (int k = 0; k < 2; ++k) {
-                            const int tok = tok0 + 2 * quad + k;
-                            if (tok >= T.ncols) break;
-                            const float f = T.shared ? inv : ctl.factor[team][tp][tok];
-                            const float4 v = make_float4(f * __uint_as_float(w[k].x), f * __uint_as_float(w[k].y),
-                                                         f * __uint_as_float(w[k].z), f * __uint_as_float(w[k].w));
-                            if (T.shared) {
-                                const size_t o = (size_t)(T.first + tok) * L.rows + col;
-                                *(float4*)(L.shexp + o) = v;
-                                if (L.l_out) {
-                                    const float4 e4 = *(const float4*)(L.residual + o);
-                                    *(float4*)(L.l_out + o) = make_float4(v.x + e4.x, v.y + e4.y, v.z + e4.z, v.w + e4.w);
-                                }
-                            } else {
-                                float* p = ctl.dst[team][tp][tok];
-                                if (p) *(float4*)(p + col) = v;
-                            }
+                    for (int k = 0; k < 4; ++k) w[k] = quad_of(buf + (4 * quad + k) * kPfTileM);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (!p[k]) continue;
+                        const float4 v = make_float4(f[k] * __uint_as_float(w[k].x), f[k] * __uint_as_float(w[k].y),
+                                                     f[k] * __uint_as_float(w[k].z), f[k] * __uint_as_float(w[k].w));
+                        *(float4*)(p[k] + col) = v;
+                        if (T.shared && L.l_out) {
+                            const size_t o = (size_t)(p[k] - L.shexp) + col;
+                            const float4 e4 = *(const float4*)(L.residual + o);
+                            *(float4*)(L.l_out + o) = make_float4(v.x + e4.x, v.y + e4.y, v.z + e4.z, v.w + e4.w);
                         }
                     }
                 }

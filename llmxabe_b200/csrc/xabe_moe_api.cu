@@ -493,7 +493,8 @@ int launch_prefill(xabe_moe* m, cudaStream_t st, PrefillLaunch& L, int qr, int q
     if (L.has_routed) box = (int)rows_box_bytes(qr == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
     if (L.has_shared) box = std::max(box, (int)rows_box_bytes(qs == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0));
     L.slot_bytes = 2 * kPfTileM * box;
-    const uint32_t smem = pf_smem_bytes(L.slot_bytes);
+    L.epi_bufs = pf_smem_bytes(L.slot_bytes, 2) <= 220u * 1024u ? 2 : 1;
+    const uint32_t smem = pf_smem_bytes(L.slot_bytes, L.epi_bufs);
     if (qr == XABE_QUANT_Q6_K)
         return qs == XABE_QUANT_Q6_K ? launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q6K>(m, st, L, smem)
                                      : launch_prefill_t<MODE, QUANT_Q6K, QUANT_Q8_0>(m, st, L, smem);
@@ -895,23 +896,23 @@ int launch_router(xabe_moe* m, cudaStream_t st, const float* router, const float
     bool regw = g.max_tokens >= 256;
     if (m->router_regw >= 0) regw = m->router_regw != 0;
     if (regw && g.max_tokens >= 2 && g.num_experts % kRwExperts == 0 && (g.hidden == 2048 || g.hidden == 1024)) {
-        // eight expert rows per CTA and two CTAs per SM (measured 0.085 against 0.091 ms at 2048 tokens);
-        // router_regw 1 selects sixteen rows and one CTA per SM
-        const int ne = m->router_regw == 1 ? 16 : 8;
-        const size_t smem_r = router_regw_smem((int)g.hidden, ne);
-        unsigned gx = g.num_experts / ne;
-        unsigned gy = (unsigned)m->sm_count * (ne == 16 ? 1u : 2u) / gx;
+        // sixteen experts per CTA, as two sets of threads that hold eight rows each (measured at 16384 tokens: see
+        // the kernel); router_regw 1 selects one set that holds sixteen
+        const int ne = m->router_regw == 1 ? 16 : 8, parts = 16 / ne;
+        const size_t smem_r = router_regw_smem((int)g.hidden, ne, parts);
+        unsigned gx = g.num_experts / 16;
+        unsigned gy = (unsigned)m->sm_count / gx;
         unsigned pairs = (g.max_tokens + kRrStageTokens - 1) / kRrStageTokens;
         if (gy < 1) gy = 1;
         if (gy > pairs) gy = pairs;
         auto go_regw = [&](auto kern) -> int {
             CUDA_TRY(allow_dynamic_smem((const void*)kern, smem_r));
-            CUDA_TRY(launch_pdl(m->pdl, kern, dim3(gx, gy), dim3(256), smem_r, st, router, (const float*)m->normed,
+            CUDA_TRY(launch_pdl(m->pdl, kern, dim3(gx, gy), dim3(256 * parts), smem_r, st, router, (const float*)m->normed,
                                 (const int*)m->valid_tokens, (int)g.num_experts, bias, m->logits, m->status));
             return XABE_OK;
         };
-        if (ne == 8) return g.hidden == 2048 ? go_regw(k_router_logits_regw<8, 8>) : go_regw(k_router_logits_regw<4, 8>);
-        return g.hidden == 2048 ? go_regw(k_router_logits_regw<8, 16>) : go_regw(k_router_logits_regw<4, 16>);
+        if (ne == 8) return g.hidden == 2048 ? go_regw(k_router_logits_regw<8, 8, 2>) : go_regw(k_router_logits_regw<4, 8, 2>);
+        return g.hidden == 2048 ? go_regw(k_router_logits_regw<8, 16, 1>) : go_regw(k_router_logits_regw<4, 16, 1>);
     }
     // wide passes: sixteen expert rows per CTA, the tokens shared out over the SMs
     if (g.max_tokens >= 32 && g.num_experts % kRwExperts == 0 && (g.hidden == 2048 || g.hidden == 1024)) {
