@@ -258,6 +258,7 @@ __device__ __forceinline__ void dense_consume(const DenseRowsLaunch& L, uint8_t*
 // grid: number of SMs; block: kDrThreads (warps 0-1 load, warps 2-17 consume).
 template <int MODE, int QUANT, int NG>
 __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L) {
+    pdl_launch_dependents();
     extern __shared__ __align__(128) uint8_t dr_raw[];
     __shared__ int abort_flag;
     uint8_t* smem = dr_raw + ((128u - (smem_u32(dr_raw) & 127u)) & 127u);
@@ -276,8 +277,6 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
     }
     __syncthreads();
     volatile int* abortp = &abort_flag;
-    const int valid = min(*L.valid_tokens, L.max_tokens);
-    if (valid <= 0) return;
     constexpr int span_b = QUANT == QUANT_Q6K ? 210 : 272;
     const int n_spans = L.k / kSpanElems;
     const size_t row_bytes = (size_t)n_spans * span_b;
@@ -298,7 +297,7 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
         constexpr int ROWS_PER_PASS = kDrLoadWarps * 2;                   // sixteen lanes per weight row
         const int wrow = LL >> 4, wpart = LL & 15;
         const int xrow = LL >> 5, xpart = LL & 31;                        // activations: thirty-two lanes per row
-        int st = 0;
+        int st = 0, valid = -1;
         uint32_t use = 0;
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
             const int rb = u / KS, ks = u - rb * KS;
@@ -336,6 +335,14 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
                             dst += dst_step;
                         }
                     }
+                    if (valid < 0) {  // the first stage's weights are on their way; the activations have a producer
+                        pdl_wait();
+                        valid = min(*L.valid_tokens, L.max_tokens);
+                        if (valid <= 0) {
+                            asm volatile("cp.async.wait_all;" ::: "memory");
+                            return;
+                        }
+                    }
                     const uint32_t x32 = slot32 + (uint32_t)(kDrStageRows * L.raw_pitch);
                     for (int tk = xrow; tk < valid; tk += kDrLoadWarps)
                         cp_async16(x32 + (uint32_t)tk * kDrXPitch + (uint32_t)xpart * 16u,
@@ -353,6 +360,9 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
     }
 
     // ---------------------------------- consumers ----------------------------------
+    pdl_wait();
+    const int valid = min(*L.valid_tokens, L.max_tokens);
+    if (valid <= 0) return;
     // As many groups as hold live tokens: a handle of 64 with 43 live ones runs the code for six groups, not for
     // eight (164 -> 149 us per layer).  The code is chosen once per launch; a bound inside the loops cost more
     // than it saved.
@@ -379,6 +389,8 @@ __global__ void __launch_bounds__(256) k_sum_k_splits(const float* __restrict__ 
                                                       const int* __restrict__ valid_tokens,
                                                       float* __restrict__ out, const float* __restrict__ residual,
                                                       float* __restrict__ l_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int tk = blockIdx.x;
     if (tk >= *valid_tokens) return;
     const int j = blockIdx.y * 256 + threadIdx.x;

@@ -63,7 +63,6 @@ __host__ __device__ inline size_t front_smem(int hidden, int tt) {
 template <int TT>
 __global__ void __launch_bounds__(kFrontThreads) k_decode_front(FrontLaunch P) {
     pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(128) float fs[];
     __shared__ __align__(8) uint64_t wbar, xbar;
     __shared__ float warp_tot[TT][32];
@@ -86,6 +85,7 @@ __global__ void __launch_bounds__(kFrontThreads) k_decode_front(FrontLaunch P) {
         mbar_expect_tx(&wbar, wbytes);
         tma_bulk_g2s(w_rows, P.router + (size_t)e0 * hidden, wbytes, &wbar);
     }
+    pdl_wait();  // (the router rows, which no kernel of this library writes, are on their way)
     const int live = *P.valid_tokens;
     // a tile without live tokens takes no ticket (the counts below are over live tiles); its router
     // rows may still be landing, and a CTA must not exit under a copy into its shared memory

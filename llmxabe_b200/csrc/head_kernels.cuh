@@ -62,6 +62,7 @@ __device__ __forceinline__ void head_half(const uint8_t* pa, const uint8_t* pb, 
 // Every wait is bounded as in k_expert_stream.
 template <int QUANT>
 __global__ void __launch_bounds__(32 * (1 + kStreamConsumerWarps), 1) k_head_rows(const __grid_constant__ HeadLaunch P) {
+    pdl_launch_dependents();
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ int abort_flag;
     uint8_t* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(32 * (1 + kStreamConsumerWarps), 1) k_head_row
     }
 
     // ---------------------------------- consumers ----------------------------------
+    pdl_wait();  // (the producer reads weights only)
     // This pass's activation rows (up to eight tokens) as hi = f16(x) and lo = f16(x - hi); rows past the
     // batch are zero.  The weight ring fills meanwhile.  (A launch of its own that wrote both parts to
     // memory first cost 5 us plus its launch; each CTA reads the same number of bytes either way.)
@@ -214,6 +216,8 @@ __device__ __forceinline__ void argmax_warp(float& best, int& idx) {
 
 __global__ void __cluster_dims__(kArgmaxSplits, 1, 1) __launch_bounds__(kArgmaxThreads)
     k_head_argmax(const float* __restrict__ logits, int vocab, int tokens, int* __restrict__ out) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float bv[32], cv[kArgmaxSplits];
     __shared__ int bi[32], ci[kArgmaxSplits];
     const int tk = blockIdx.x / kArgmaxSplits, part = blockIdx.x % kArgmaxSplits;  // part: the CTA's rank in its cluster

@@ -404,7 +404,6 @@ __device__ __forceinline__ int gateup_span_of(int w, int h, int n_spans) {
 template <int MODE, int QR, int QS, bool TAIL = false>
 __global__ void __launch_bounds__(kStreamThreads, 1) k_expert_stream(StreamLaunch L) {
     pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int abort_flag;
     __shared__ StreamPlan plan_shared;  // computed once, by thread 0
@@ -429,6 +428,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_expert_stream(StreamLaunc
         }
         fence_mbar_init();
     }
+    pdl_wait();
     if (threadIdx.x == 0) plan_shared = stream_plan(L, ROWS_PER_TILE);
     __syncthreads();
     const StreamPlan plan = plan_shared;

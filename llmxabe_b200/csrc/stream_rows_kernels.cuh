@@ -73,7 +73,6 @@ __device__ __forceinline__ void tma_load_box_2d(void* dst, const CUtensorMap* tm
 template <int QR, int QS>
 __global__ void __launch_bounds__(kStreamThreads, 1) k_gateup_rows(const __grid_constant__ RowsLaunch P) {
     pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ int abort_flag;
     const StreamLaunch& L = P.L;
@@ -97,6 +96,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) k_gateup_rows(const __grid_
         }
         fence_mbar_init();
     }
+    pdl_wait();
     __syncthreads();
     volatile int* abortp = &abort_flag;
     const int n_spans = L.k / kSpanElems;

@@ -74,13 +74,24 @@ cudaError_t allow_dynamic_smem(const void* kern, size_t needed) {
     return cudaSuccess;
 }
 
-// Launch, optionally with programmatic stream serialization (the kernel may then be scheduled while
-// its predecessor on the stream drains; every kernel launched through here waits for the predecessor
-// before it touches its output, see pdl_wait()).  Per handle, off unless XABE_TUNE_PDL was set.
+// Launch with programmatic stream serialization where that pays (the kernel may then be scheduled while its
+// predecessor on the stream drains; every kernel launched through here waits for the predecessor before it
+// touches anything but constant weights, see pdl_wait()): on streams that are not being captured, where it
+// hides launch latency (one layer of 1 / 3 / 64 tokens: 38.4 / 55.3 / 164 -> 35.0 / 49.4 / 160 us).  Inside a replayed
+// graph the launches are ready anyway and the early CTAs only take room from the running kernel (40 layers
+// of one token: 1383 -> 1562 us), so there it is off unless XABE_TUNE_PDL was set.
+bool is_eager(cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cs == cudaStreamCaptureStatusNone;
+}
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                        Args&&... args) {
-    const bool off = !pdl;
+    const bool off = !pdl && !is_eager(st);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -507,8 +518,7 @@ template <int MODE, int QUANT>
 int launch_dense_rows_q(xabe_moe* m, cudaStream_t st, const DenseRowsLaunch& P, int ng, uint32_t smem) {
     auto go = [&](auto kern) -> int {
         CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-        kern<<<dim3(m->sm_count), dim3(kDrThreads), smem, counted(st)>>>(P);
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(launch_pdl(m->pdl, kern, dim3(m->sm_count), dim3(kDrThreads), smem, st, P));
         return XABE_OK;
     };
     switch (ng) {
@@ -674,10 +684,9 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
             smem = shape(qd);
             if ((rc = launch_dense_rows<MODE_DOWN>(m, st, P, qd, ng, smem))) return rc;
             if (P.k_splits > 1) {
-                k_sum_k_splits<<<dim3(g.max_tokens, (g.hidden + 255) / 256), 256, 0, counted(st)>>>(
-                    m->dense_partial, P.k_splits, (int)g.max_tokens, (int)g.hidden, m->valid_tokens, shexp_out,
-                    dense ? dense->residual : nullptr, dense ? dense->l_out : nullptr);
-                CUDA_TRY(cudaGetLastError());
+                CUDA_TRY(launch_pdl(m->pdl, k_sum_k_splits, dim3(g.max_tokens, (g.hidden + 255) / 256), dim3(256), 0, st,
+                                    m->dense_partial, P.k_splits, (int)g.max_tokens, (int)g.hidden, m->valid_tokens,
+                                    shexp_out, dense ? dense->residual : nullptr, dense ? dense->l_out : nullptr));
                 if (dense) dense->done = true;
             }
             return XABE_OK;
@@ -2201,12 +2210,11 @@ int xabe_lm_head_forward(xabe_lm_head* m, void* stream, xabe_quant_tensor weight
     const dim3 grid(m->sm_count, (tokens + 7) / 8), block(32 * (1 + kStreamConsumerWarps));
     if (q == QUANT_Q6K) {
         CUDA_TRY(allow_dynamic_smem((const void*)k_head_rows<QUANT_Q6K>, smem));
-        k_head_rows<QUANT_Q6K><<<grid, block, smem, counted(st)>>>(P);
+        CUDA_TRY(launch_pdl(false, k_head_rows<QUANT_Q6K>, grid, block, smem, st, P));
     } else {
         CUDA_TRY(allow_dynamic_smem((const void*)k_head_rows<QUANT_Q8_0>, smem));
-        k_head_rows<QUANT_Q8_0><<<grid, block, smem, counted(st)>>>(P);
+        CUDA_TRY(launch_pdl(false, k_head_rows<QUANT_Q8_0>, grid, block, smem, st, P));
     }
-    CUDA_TRY(cudaGetLastError());
     return XABE_OK;
 }
 
@@ -2220,8 +2228,8 @@ int xabe_lm_head_argmax(xabe_lm_head* m, void* stream, const float* logits, size
         return fail(XABE_ERR_BUFFER_LENGTH, "logits must hold %zu floats, holds %zu",
                     (size_t)m->g.max_tokens * m->g.vocab, logits_len);
     if (tokens == 0) return XABE_OK;
-    k_head_argmax<<<tokens * kArgmaxSplits, kArgmaxThreads, 0, counted((cudaStream_t)stream)>>>(logits, (int)m->g.vocab, tokens, out);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_pdl(false, k_head_argmax, dim3(tokens * kArgmaxSplits), dim3(kArgmaxThreads), 0, (cudaStream_t)stream,
+                        logits, (int)m->g.vocab, tokens, out));
     return XABE_OK;
 }
 
