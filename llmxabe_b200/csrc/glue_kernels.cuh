@@ -643,6 +643,8 @@ __global__ void __launch_bounds__(32) k_align_count(const int* __restrict__ topk
                                                     int block_capacity, int* __restrict__ chunk_hist,
                                                     int* __restrict__ sorted_token_ids,
                                                     int* __restrict__ expert_ids) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ int hist[];
     int c = blockIdx.x, lane = threadIdx.x;
     int numel = *valid_tokens * top_k;
@@ -669,6 +671,8 @@ __global__ void k_align_scan(int num_experts, int n_chunks, int block_size, int*
                              int* __restrict__ expert_offsets, int* __restrict__ expert_counts,
                              int* __restrict__ expert_ids, int* __restrict__ num_tokens_post_pad,
                              int* __restrict__ group_base, int* __restrict__ n_work) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ int warp_sums[33];
     int e = threadIdx.x;
     int total = 0;
@@ -741,6 +745,8 @@ __global__ void __launch_bounds__(32) k_align_scatter(const int* __restrict__ to
                                                       const int* __restrict__ group_base,
                                                       const float* __restrict__ topk_weights,
                                                       int* __restrict__ work_items) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ int cursor[];
     int c = blockIdx.x, lane = threadIdx.x;
     int numel = *valid_tokens * top_k;
@@ -1212,6 +1218,8 @@ __global__ void __launch_bounds__(256) k_ep_combine(
 __global__ void __launch_bounds__(256) k_add_residual(const float* __restrict__ ffn, const float* __restrict__ residual,
                                                       const int* __restrict__ valid_tokens, int hidden,
                                                       float* __restrict__ l_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     if (t >= *valid_tokens) return;
     const size_t base = (size_t)t * hidden;
@@ -1234,6 +1242,8 @@ __global__ void __launch_bounds__(256) k_add_residual(const float* __restrict__ 
 // exact (crates/xabe-kernels/src/quant.rs:1350-1358 pins the same for tensors).
 __global__ void k_rows_bf16_to_f32(const unsigned short* __restrict__ x, float* __restrict__ out,
                                    const int* __restrict__ valid_tokens, int width) {
+    pdl_launch_dependents();
+    pdl_wait();
     int row = blockIdx.x;
     if (row >= *valid_tokens) return;
     size_t base = (size_t)row * width;

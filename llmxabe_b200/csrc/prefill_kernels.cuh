@@ -260,6 +260,8 @@ __device__ __forceinline__ bool warp_wait_pf(uint64_t* bar, uint32_t parity, vol
 __global__ void k_build_prefill_items(int num_experts, const int* __restrict__ expert_offsets,
                                       const int* __restrict__ expert_counts, int* __restrict__ items,
                                       int* __restrict__ n_items, int item_cols) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ int warp_sums[33];
     int e = threadIdx.x;
     const int mine = e < num_experts ? (expert_counts[e] + item_cols - 1) / item_cols : 0;
@@ -464,13 +466,10 @@ __host__ __device__ inline uint32_t pf_smem_bytes(int slot_bytes, int epi_bufs) 
 // grid: one CTA per SM; block kPfThreads.
 template <int MODE, int QR, int QS>
 __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_constant__ PrefillLaunch L) {
+    pdl_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) PfCtl ctl;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int valid = *L.valid_tokens;
-    const int n_routed = L.has_routed ? *L.n_items : 0;
-    const int n_shared = L.has_shared ? (valid + kPfTileN - 1) / kPfTileN : 0;
-    const int n_tiles = (n_routed + n_shared) * L.row_units;
     const int n_spans = L.k / kSpanElems;
     uint8_t* bst = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* epi = bst + (size_t)kPfStages * kPfBStageBytes;
@@ -498,6 +497,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) k_prefill_gemm(const __grid_con
         tmem_alloc(&ctl.tmem_base, 512);  // 256 columns of accumulators, 256 of weights
         tmem_relinquish();
     }
+    pdl_wait();
+    const int valid = *L.valid_tokens;
+    const int n_routed = L.has_routed ? *L.n_items : 0;
+    const int n_shared = L.has_shared ? (valid + kPfTileN - 1) / kPfTileN : 0;
+    const int n_tiles = (n_routed + n_shared) * L.row_units;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

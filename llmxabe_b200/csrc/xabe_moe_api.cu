@@ -80,6 +80,7 @@ cudaError_t allow_dynamic_smem(const void* kern, size_t needed) {
 // hides launch latency (one layer of 1 / 3 / 64 tokens: 38.4 / 55.3 / 164 -> 35.0 / 49.4 / 160 us).  Inside a replayed
 // graph the launches are ready anyway and the early CTAs only take room from the running kernel (40 layers
 // of one token: 1383 -> 1562 us), so there it is off unless XABE_TUNE_PDL was set.
+enum class Overlap { never, eager, always };
 bool is_eager(cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
@@ -89,9 +90,9 @@ bool is_eager(cudaStream_t st) {
     return cs == cudaStreamCaptureStatusNone;
 }
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+cudaError_t launch_pdl(Overlap overlap, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                        Args&&... args) {
-    const bool off = !pdl && !is_eager(st);
+    const bool off = overlap == Overlap::never || (overlap == Overlap::eager && !is_eager(st));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -177,6 +178,7 @@ struct xabe_moe {
     int sm_count = 0;
     cudaStream_t side = nullptr;     // the shared expert beside the dispatch (see forks_shared)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    bool plain_launches = false;     // no overlap of launches during this call (see block_forward)
     int grid_limit = 0;              // > 0: the streaming kernels' grid, while a launch shares the GPU
     int* pf_items = nullptr;    // token tiles for the tcgen05 prefill kernels
     int* pf_n_items = nullptr;
@@ -227,6 +229,13 @@ struct xabe_moe {
 };
 
 namespace {
+
+// Prefill widths keep plain launches: their kernels fill the GPU, and a persistent CTA that starts early takes
+// its SM from them (2048 tokens: 472 us, with overlapped launches 497).
+inline Overlap overlap_of(const xabe_moe* m) {
+    if (m->plain_launches || (!m->pdl && m->g.max_tokens >= kPrefillMinTokens)) return Overlap::never;
+    return m->pdl ? Overlap::always : Overlap::eager;
+}
 
 constexpr int kProfCalls = 256;
 
@@ -344,7 +353,7 @@ int launch_stream_t(xabe_moe* m, cudaStream_t st, const StreamLaunch& L, uint32_
     auto kern = (MODE == MODE_DOWN && L.tail_done) ? k_expert_stream<MODE, QR, QS, MODE == MODE_DOWN>
                                                    : k_expert_stream<MODE, QR, QS, false>;
     CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-    CUDA_TRY(launch_pdl(m->pdl, kern, dim3(stream_grid(m)), dim3(kStreamThreads), smem, st, L));
+    CUDA_TRY(launch_pdl(overlap_of(m), kern, dim3(stream_grid(m)), dim3(kStreamThreads), smem, st, L));
     return XABE_OK;
 }
 
@@ -444,7 +453,7 @@ template <int QR, int QS>
 int launch_rows_t(xabe_moe* m, cudaStream_t st, const RowsLaunch& P, uint32_t smem) {
     auto kern = k_gateup_rows<QR, QS>;
     CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-    CUDA_TRY(launch_pdl(m->pdl, kern, dim3(stream_grid(m)), dim3(kStreamThreads), smem, st, P));
+    CUDA_TRY(launch_pdl(overlap_of(m), kern, dim3(stream_grid(m)), dim3(kStreamThreads), smem, st, P));
     return XABE_OK;
 }
 
@@ -493,8 +502,7 @@ template <int MODE, int QR, int QS>
 int launch_prefill_t(xabe_moe* m, cudaStream_t st, const PrefillLaunch& L, uint32_t smem) {
     auto kern = k_prefill_gemm<MODE, QR, QS>;
     CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-    kern<<<m->sm_count, kPfThreads, smem, counted(st)>>>(L);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_pdl(overlap_of(m), kern, dim3(m->sm_count), dim3(kPfThreads), smem, st, L));
     return XABE_OK;
 }
 template <int MODE>
@@ -518,7 +526,7 @@ template <int MODE, int QUANT>
 int launch_dense_rows_q(xabe_moe* m, cudaStream_t st, const DenseRowsLaunch& P, int ng, uint32_t smem) {
     auto go = [&](auto kern) -> int {
         CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-        CUDA_TRY(launch_pdl(m->pdl, kern, dim3(m->sm_count), dim3(kDrThreads), smem, st, P));
+        CUDA_TRY(launch_pdl(overlap_of(m), kern, dim3(m->sm_count), dim3(kDrThreads), smem, st, P));
         return XABE_OK;
     };
     switch (ng) {
@@ -684,7 +692,8 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
             smem = shape(qd);
             if ((rc = launch_dense_rows<MODE_DOWN>(m, st, P, qd, ng, smem))) return rc;
             if (P.k_splits > 1) {
-                CUDA_TRY(launch_pdl(m->pdl, k_sum_k_splits, dim3(g.max_tokens, (g.hidden + 255) / 256), dim3(256), 0, st,
+                CUDA_TRY(launch_pdl(overlap_of(m), k_sum_k_splits, dim3(g.max_tokens, (g.hidden + 255) / 256),
+                                    dim3(256), 0, st,
                                     m->dense_partial, P.k_splits, (int)g.max_tokens, (int)g.hidden, m->valid_tokens,
                                     shexp_out, dense ? dense->residual : nullptr, dense ? dense->l_out : nullptr));
                 if (dense) dense->done = true;
@@ -877,7 +886,7 @@ int launch_rms_norm(xabe_moe* m, cudaStream_t st, const float* x, const float* w
     if (!gate_w && ept <= 8) {
         const dim3 grid((unsigned)std::min<uint32_t>(m->g.max_tokens, 2u * (uint32_t)m->sm_count));
         auto go = [&](auto kern) -> int {
-            CUDA_TRY(launch_pdl(m->pdl, kern, grid, dim3(block), 0, st, x, weight, m->normed, m->normed_h,
+            CUDA_TRY(launch_pdl(overlap_of(m), kern, grid, dim3(block), 0, st, x, weight, m->normed, m->normed_h,
                                 (const int*)m->valid_tokens, (int)m->g.hidden, m->eps));
             return XABE_OK;
         };
@@ -892,7 +901,7 @@ int launch_rms_norm(xabe_moe* m, cudaStream_t st, const float* x, const float* w
             default: return go(k_rms_norm_stream<8>);
         }
     }
-    CUDA_TRY(launch_pdl(m->pdl, k_rms_norm, dim3(m->g.max_tokens), dim3(block), smem, st, x, weight, m->normed,
+    CUDA_TRY(launch_pdl(overlap_of(m), k_rms_norm, dim3(m->g.max_tokens), dim3(block), smem, st, x, weight, m->normed,
                         m->normed_h, m->valid_tokens, (int)m->g.hidden, m->eps, gate_w, m->gate));
     return XABE_OK;
 }
@@ -916,7 +925,8 @@ int launch_router(xabe_moe* m, cudaStream_t st, const float* router, const float
         if (gy > pairs) gy = pairs;
         auto go_regw = [&](auto kern) -> int {
             CUDA_TRY(allow_dynamic_smem((const void*)kern, smem_r));
-            CUDA_TRY(launch_pdl(m->pdl, kern, dim3(gx, gy), dim3(256 * parts), smem_r, st, router, (const float*)m->normed,
+            CUDA_TRY(launch_pdl(overlap_of(m), kern, dim3(gx, gy), dim3(256 * parts), smem_r, st, router, (const
+                                float*)m->normed,
                                 (const int*)m->valid_tokens, (int)g.num_experts, bias, m->logits, m->status));
             return XABE_OK;
         };
@@ -933,7 +943,8 @@ int launch_router(xabe_moe* m, cudaStream_t st, const float* router, const float
         if (gy > tiles) gy = tiles;
         auto go_wide = [&](auto kern) -> int {
             CUDA_TRY(allow_dynamic_smem((const void*)kern, smem_w));
-            CUDA_TRY(launch_pdl(m->pdl, kern, dim3(gx, gy), dim3(256), smem_w, st, router, (const float*)m->normed,
+            CUDA_TRY(launch_pdl(overlap_of(m), kern, dim3(gx, gy), dim3(256), smem_w, st, router, (const
+                                float*)m->normed,
                                 (const int*)m->valid_tokens, (int)g.num_experts, bias, m->logits, m->status));
             return XABE_OK;
         };
@@ -950,7 +961,7 @@ int launch_router(xabe_moe* m, cudaStream_t st, const float* router, const float
         int tiles_per_cta = g.max_tokens > 128 ? 8 : 1;
         unsigned ty = (g.max_tokens + tt * tiles_per_cta - 1) / (tt * tiles_per_cta);
         CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-        CUDA_TRY(launch_pdl(m->pdl, kern, dim3(ex, ty), block, smem, st, router, (const float*)m->normed,
+        CUDA_TRY(launch_pdl(overlap_of(m), kern, dim3(ex, ty), block, smem, st, router, (const float*)m->normed,
                             (const int*)m->valid_tokens, (int)g.hidden, (int)g.num_experts, bias, m->logits,
                             tiles_per_cta, m->status));
         return XABE_OK;
@@ -971,51 +982,48 @@ int launch_route_and_dispatch(xabe_moe* m, cudaStream_t st, const float* logits)
         const size_t smem = dispatch_small_smem((int)g.num_experts);
         const float* fused_logits = logits;
         if (logits && g.max_tokens > 8) {  // route on many SMs first
-            CUDA_TRY(launch_pdl(m->pdl, k_route, dim3((g.max_tokens + 7) / 8), dim3(256), 0, st, logits,
+            CUDA_TRY(launch_pdl(overlap_of(m), k_route, dim3((g.max_tokens + 7) / 8), dim3(256), 0, st, logits,
                                 (const int*)m->valid_tokens, (int)g.num_experts, (int)g.experts_per_token,
                                 m->topk_ids, m->topk_weights));
             fused_logits = nullptr;
         }
-        CUDA_TRY(launch_pdl(m->pdl, k_route_dispatch_small, dim3(1), dim3(kDispatchThreads), smem, st, fused_logits,
+        CUDA_TRY(launch_pdl(overlap_of(m), k_route_dispatch_small, dim3(1), dim3(kDispatchThreads), smem, st,
+                            fused_logits,
                             (const int*)m->valid_tokens, (int)g.num_experts, (int)g.experts_per_token,
                             (int)g.block_size, (int)m->sorted_capacity, (int)m->block_capacity, m->topk_ids,
                             m->topk_weights, m->sorted_token_ids, m->expert_ids, m->num_tokens_post_pad,
                             m->expert_offsets, m->expert_counts, m->work_items, m->n_work));
         if (prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate)) {  // few experts, many tokens
             int threads = ((int)g.num_experts + 31) / 32 * 32;
-            k_build_prefill_items<<<1, threads, hist_bytes, counted(st)>>>((int)g.num_experts, m->expert_offsets,
-                                                                  m->expert_counts, m->pf_items, m->pf_n_items, kPfTileN);
-            CUDA_TRY(cudaGetLastError());
+            CUDA_TRY(launch_pdl(overlap_of(m), k_build_prefill_items, dim3(1), dim3(threads), hist_bytes, st,
+                                (int)g.num_experts, m->expert_offsets, m->expert_counts, m->pf_items, m->pf_n_items,
+                                kPfTileN));
         }
         return XABE_OK;
     }
     if (logits) {
-        k_route<<<(g.max_tokens + 7) / 8, 256, 0, counted(st)>>>(logits, m->valid_tokens, (int)g.num_experts,
-                                                       (int)g.experts_per_token, m->topk_ids, m->topk_weights);
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(launch_pdl(overlap_of(m), k_route, dim3((g.max_tokens + 7) / 8), dim3(256), 0, st, logits,
+                            m->valid_tokens, (int)g.num_experts, (int)g.experts_per_token, m->topk_ids,
+                            m->topk_weights));
     }
-    k_align_count<<<m->n_chunks, 32, hist_bytes, counted(st)>>>(m->topk_ids, m->valid_tokens, (int)g.experts_per_token,
-                                                      (int)g.num_experts, m->n_chunks, m->align_chunk, (int)m->sorted_capacity,
-                                                      (int)m->block_capacity, m->chunk_hist,
-                                                      m->sorted_token_ids, m->expert_ids);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_pdl(overlap_of(m), k_align_count, dim3(m->n_chunks), dim3(32), hist_bytes, st, m->topk_ids,
+                        m->valid_tokens, (int)g.experts_per_token, (int)g.num_experts, m->n_chunks, m->align_chunk,
+                        (int)m->sorted_capacity, (int)m->block_capacity, m->chunk_hist, m->sorted_token_ids,
+                        m->expert_ids));
     // Only the work list of the kernels that will run: the regime must be chosen before this call.
     const bool tc = prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate);
     int threads = ((int)g.num_experts + 31) / 32 * 32;
-    k_align_scan<<<1, threads, 0, counted(st)>>>((int)g.num_experts, m->n_chunks, (int)g.block_size,
-                                                 m->chunk_hist, m->expert_offsets, m->expert_counts,
-                                                 m->expert_ids, m->num_tokens_post_pad, m->group_base,
-                                                 tc ? nullptr : m->n_work);
-    CUDA_TRY(cudaGetLastError());
-    k_align_scatter<<<m->n_chunks, 32, hist_bytes, counted(st)>>>(
-        m->topk_ids, m->valid_tokens, (int)g.experts_per_token, (int)g.num_experts, m->align_chunk, m->chunk_hist,
-        m->expert_offsets, m->sorted_token_ids, m->expert_counts, m->group_base, m->topk_weights,
-        tc ? nullptr : m->work_items);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_pdl(overlap_of(m), k_align_scan, dim3(1), dim3(threads), 0, st, (int)g.num_experts, m->n_chunks,
+                        (int)g.block_size, m->chunk_hist, m->expert_offsets, m->expert_counts, m->expert_ids,
+                        m->num_tokens_post_pad, m->group_base, tc ? nullptr : m->n_work));
+    CUDA_TRY(launch_pdl(overlap_of(m), k_align_scatter, dim3(m->n_chunks), dim3(32), hist_bytes, st, m->topk_ids,
+                        m->valid_tokens, (int)g.experts_per_token, (int)g.num_experts, m->align_chunk, m->chunk_hist,
+                        m->expert_offsets, m->sorted_token_ids, m->expert_counts, m->group_base, m->topk_weights, tc ?
+                        nullptr : m->work_items));
     if (tc) {
-        k_build_prefill_items<<<1, threads, hist_bytes, counted(st)>>>((int)g.num_experts, m->expert_offsets,
-                                                              m->expert_counts, m->pf_items, m->pf_n_items, kPfTileN);
-        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(launch_pdl(overlap_of(m), k_build_prefill_items, dim3(1), dim3(threads), hist_bytes, st,
+                            (int)g.num_experts, m->expert_offsets, m->expert_counts, m->pf_items, m->pf_n_items,
+                            kPfTileN));
     }
     return XABE_OK;
 }
@@ -1082,7 +1090,7 @@ int launch_front(xabe_moe* m, cudaStream_t st, const float* x, const xabe_moe_la
     const dim3 grid((g.num_experts + 3) / 4, (g.max_tokens + tt - 1) / tt);
     auto go = [&](auto kern) -> int {
         CUDA_TRY(allow_dynamic_smem((const void*)kern, smem));
-        CUDA_TRY(launch_pdl(m->pdl, kern, grid, dim3(kFrontThreads), smem, st, P));
+        CUDA_TRY(launch_pdl(overlap_of(m), kern, grid, dim3(kFrontThreads), smem, st, P));
         return XABE_OK;
     };
     int rc = tt == 8 ? go(k_decode_front<8>) : tt == 4 ? go(k_decode_front<4>) : go(k_decode_front<1>);
@@ -1090,7 +1098,8 @@ int launch_front(xabe_moe* m, cudaStream_t st, const float* x, const xabe_moe_la
     if (!with_routing) return launch_route_and_dispatch(m, st, m->logits);
     if (P.fused_dispatch) return rc;
     // wider handles: the tables from the routing the launch above stored (256 threads, one CTA)
-    CUDA_TRY(launch_pdl(m->pdl, k_route_dispatch_small, dim3(1), dim3(kDispatchThreads), dispatch_small_smem((int)g.num_experts),
+    CUDA_TRY(launch_pdl(overlap_of(m), k_route_dispatch_small, dim3(1), dim3(kDispatchThreads),
+                        dispatch_small_smem((int)g.num_experts),
                         st, (const float*)nullptr, (const int*)m->valid_tokens, (int)g.num_experts,
                         (int)g.experts_per_token, (int)g.block_size, (int)m->sorted_capacity, (int)m->block_capacity,
                         m->topk_ids, m->topk_weights, m->sorted_token_ids, m->expert_ids, m->num_tokens_post_pad,
@@ -1332,7 +1341,7 @@ int xabe_moe_gate_and_combine(xabe_moe* m, void* stream, const float* shared_gat
     if (residual_len != n || ffn_out_len != n || l_out_len != n)
         return fail(XABE_ERR_BUFFER_LENGTH, "gate_and_combine buffers must hold %zu floats", n);
     dim3 grid(g.max_tokens, g.max_tokens >= 512 ? 1u : (g.hidden + 255) / 256);
-    CUDA_TRY(launch_pdl(m->pdl,
+    CUDA_TRY(launch_pdl(overlap_of(m),
                         combine_vec(m, grid, residual, ffn_out, l_out) ? k_gate_and_combine<true> : k_gate_and_combine<false>,
                         grid, dim3(256), 0, (cudaStream_t)stream, shared_gate_inp,
                         (const float*)m->normed, (const float*)m->partial, (const float*)m->shexp, residual,
@@ -1646,6 +1655,13 @@ int xabe_moe_block_forward(xabe_moe* m, void* stream, const xabe_moe_layer_weigh
     s.up = w->shared_up;
     s.down = w->shared_down;
     const bool fork = !fused_tail && !fused_front && forks_shared(m, w);
+    // Beside the multi-launch dispatch of wide handles the early CTAs of the shared expert's kernels take SMs from
+    // it (333 tokens: 346 us with plain launches, 361 with overlapped ones; 100 tokens: 224, 208).
+    struct Plain {
+        bool& flag;
+        ~Plain() { flag = false; }
+    } plain{m->plain_launches};
+    m->plain_launches = fork && (uint64_t)g.max_tokens * g.experts_per_token > (uint64_t)kSmallPairs;
     auto fork_shared = [&]() -> int {  // the normalised rows are enqueued: the shared expert may follow them
         CUDA_TRY(cudaEventRecord(m->ev_fork, st));
         CUDA_TRY(cudaStreamWaitEvent(m->side, m->ev_fork, 0));
@@ -1682,7 +1698,7 @@ int xabe_moe_block_forward(xabe_moe* m, void* stream, const xabe_moe_layer_weigh
         if (rc) return rc;
         prof_mark(m, st, 5);
         dim3 grid(g.max_tokens, g.max_tokens >= 512 ? 1u : (g.hidden + 255) / 256);
-        CUDA_TRY(launch_pdl(m->pdl,
+        CUDA_TRY(launch_pdl(overlap_of(m),
                             combine_vec(m, grid, residual, ffn_out, l_out) ? k_gate_and_combine<true>
                                                                            : k_gate_and_combine<false>,
                             grid, dim3(256), 0, st, w->shared_gate_inp,
@@ -1769,9 +1785,8 @@ int xabe_moe_block_forward_typed(xabe_moe* m, void* stream, const xabe_moe_layer
                     g.max_tokens);
     int rc = xabe_moe_set_valid_tokens(m, stream, tokens);
     if (rc) return rc;
-    k_rows_bf16_to_f32<<<g.max_tokens, 256, 0, counted((cudaStream_t)stream)>>>((const unsigned short*)residual, m->stage_in,
-                                                                      m->valid_tokens, (int)g.hidden);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_pdl(overlap_of(m), k_rows_bf16_to_f32, dim3(g.max_tokens), dim3(256), 0, (cudaStream_t)stream,
+                        (const unsigned short*)residual, m->stage_in, m->valid_tokens, (int)g.hidden));
     return xabe_moe_block_forward(m, stream, w, m->stage_in, n, tokens, ffn_out, ffn_out_len, l_out, l_out_len);
 }
 
@@ -1801,9 +1816,8 @@ int xabe_dense_ffn_block_forward(xabe_moe* m, void* stream, const float* post_no
     DenseTail tail{residual, l_out};
     if ((rc = run_experts(m, st, MlpWeights{}, s, ffn_out, -1, nullptr, &tail))) return rc;
     if (tail.done) return XABE_OK;
-    k_add_residual<<<dim3(g.max_tokens, (g.hidden + 1023) / 1024), 256, 0, counted(st)>>>(
-        ffn_out, residual, m->valid_tokens, (int)g.hidden, l_out);
-    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(launch_pdl(overlap_of(m), k_add_residual, dim3(g.max_tokens, (g.hidden + 1023) / 1024), dim3(256), 0, st,
+                        ffn_out, residual, m->valid_tokens, (int)g.hidden, l_out));
     return XABE_OK;
 }
 
@@ -2210,10 +2224,10 @@ int xabe_lm_head_forward(xabe_lm_head* m, void* stream, xabe_quant_tensor weight
     const dim3 grid(m->sm_count, (tokens + 7) / 8), block(32 * (1 + kStreamConsumerWarps));
     if (q == QUANT_Q6K) {
         CUDA_TRY(allow_dynamic_smem((const void*)k_head_rows<QUANT_Q6K>, smem));
-        CUDA_TRY(launch_pdl(false, k_head_rows<QUANT_Q6K>, grid, block, smem, st, P));
+        CUDA_TRY(launch_pdl(Overlap::eager, k_head_rows<QUANT_Q6K>, grid, block, smem, st, P));
     } else {
         CUDA_TRY(allow_dynamic_smem((const void*)k_head_rows<QUANT_Q8_0>, smem));
-        CUDA_TRY(launch_pdl(false, k_head_rows<QUANT_Q8_0>, grid, block, smem, st, P));
+        CUDA_TRY(launch_pdl(Overlap::eager, k_head_rows<QUANT_Q8_0>, grid, block, smem, st, P));
     }
     return XABE_OK;
 }
@@ -2228,7 +2242,7 @@ int xabe_lm_head_argmax(xabe_lm_head* m, void* stream, const float* logits, size
         return fail(XABE_ERR_BUFFER_LENGTH, "logits must hold %zu floats, holds %zu",
                     (size_t)m->g.max_tokens * m->g.vocab, logits_len);
     if (tokens == 0) return XABE_OK;
-    CUDA_TRY(launch_pdl(false, k_head_argmax, dim3(tokens * kArgmaxSplits), dim3(kArgmaxThreads), 0, (cudaStream_t)stream,
+    CUDA_TRY(launch_pdl(Overlap::eager, k_head_argmax, dim3(tokens * kArgmaxSplits), dim3(kArgmaxThreads), 0, (cudaStream_t)stream,
                         logits, (int)m->g.vocab, tokens, out));
     return XABE_OK;
 }
