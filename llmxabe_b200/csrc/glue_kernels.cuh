@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(256 * PARTS, 1) k_router_logits_regw(const flo
 template <int kRouteLaneExperts>
 __device__ __forceinline__ void route_one_token(const float* __restrict__ row, int num_experts, int top_k,
                                                 int lane, int* __restrict__ ids_out,
-                                                float* __restrict__ w_out) {
+                                                float* __restrict__ w_out, int* ids_s = nullptr,
+                                                float* w_s = nullptr) {
     // the row may have been written by other CTAs of the same launch: read it through L2
     float lg[kRouteLaneExperts];
     float mx = __ldcg(row);
@@ -602,8 +603,13 @@ __device__ __forceinline__ void route_one_token(const float* __restrict__ row, i
         sel_sum += bv;  // selection order, as router.rs:62
     }
     if (lane < top_k) {
+        const float wt = sel_sum > 0.0f ? __fdiv_rn(my_sel, sel_sum) : __fdiv_rn(1.0f, (float)top_k);
         ids_out[lane] = my_id;
-        w_out[lane] = sel_sum > 0.0f ? __fdiv_rn(my_sel, sel_sum) : __fdiv_rn(1.0f, (float)top_k);
+        w_out[lane] = wt;
+        if (ids_s) {
+            ids_s[lane] = my_id;
+            w_s[lane] = wt;
+        }
     }
 }
 
@@ -634,8 +640,11 @@ __global__ void __launch_bounds__(256) k_route(const float* __restrict__ logits,
 // valid_tokens * top_k (dispatch.rs:24-26), inactive blocks are -1.
 // ---------------------------------------------------------------------------
 // Flat pairs per chunk (one warp each): small chunks put more warps to work, large ones keep the
-// one-thread-per-expert scan over the chunks short.
-__host__ __device__ inline int align_chunk_pairs(uint64_t pairs) { return pairs <= 65536 ? 256 : 1024; }
+// one-thread-per-expert scan over the chunks short.  (333 tokens, 2664 pairs: the scatter takes 10.2 us with
+// chunks of 256, 4 us with 64.)
+__host__ __device__ inline int align_chunk_pairs(uint64_t pairs) {
+    return pairs <= 8192 ? 64 : pairs <= 65536 ? 256 : 1024;
+}
 
 __global__ void __launch_bounds__(32) k_align_count(const int* __restrict__ topk_ids,
                                                     const int* __restrict__ valid_tokens, int top_k,
@@ -874,6 +883,7 @@ __device__ __forceinline__ void dispatch_tiny_warp(
 // `logits` NULL = the routing was done by k_route already.  block kDispatchThreads.
 // ---------------------------------------------------------------------------
 constexpr int kDispatchThreads = 512;
+constexpr int kDispatchRouted = 8;  // tokens it routes itself
 __host__ __device__ inline size_t dispatch_small_smem(int num_experts) {
     return (size_t)(kDispatchThreads / 32 + 3) * num_experts * sizeof(int);
 }
@@ -888,6 +898,9 @@ __global__ void __launch_bounds__(kDispatchThreads) k_route_dispatch_small(
     pdl_wait();
     extern __shared__ int sm[];
     __shared__ int warp_sums[33];
+    // what this launch routed itself, so that it is not read back through L2
+    __shared__ int ids_s[kDispatchRouted * 16];
+    __shared__ float wts_s[kDispatchRouted * 16];
     constexpr int NT = kDispatchThreads, NW = NT / 32, NB = kSmallPairs / NT;
     const int E = num_experts;
     int* hist = sm;               // [NW][E] per-warp counts, then their exclusive prefixes over the warps
@@ -896,15 +909,12 @@ __global__ void __launch_bounds__(kDispatchThreads) k_route_dispatch_small(
     int* gbase_s = start_s + E;   // [E]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int live = *valid_tokens, numel = live * top_k;
-    if (logits) {  // one token per warp; wider steps route in k_route first
-        for (int t = warp; t < live; t += NW) {
-            if (E <= 256)
-                route_one_token<8>(logits + (size_t)t * E, E, top_k, lane, topk_ids + (size_t)t * top_k,
-                                   topk_weights + (size_t)t * top_k);
-            else
-                route_one_token<16>(logits + (size_t)t * E, E, top_k, lane, topk_ids + (size_t)t * top_k,
-                                    topk_weights + (size_t)t * top_k);
-        }
+    if (logits && warp < live) {  // one token per warp, at most kDispatchRouted; wider steps route in k_route first
+        const size_t o = (size_t)warp * top_k;
+        if (E <= 256)
+            route_one_token<8>(logits + (size_t)warp * E, E, top_k, lane, topk_ids + o, topk_weights + o, ids_s + o, wts_s + o);
+        else
+            route_one_token<16>(logits + (size_t)warp * E, E, top_k, lane, topk_ids + o, topk_weights + o, ids_s + o, wts_s + o);
     }
     for (int i = tid; i < NW * E; i += NT) hist[i] = 0;
     for (int i = tid; i < sorted_capacity; i += NT) sorted_token_ids[i] = numel;
@@ -919,8 +929,8 @@ __global__ void __launch_bounds__(kDispatchThreads) k_route_dispatch_small(
     for (int b = 0; b < NB; ++b) {
         const int i = warp * chunk + 32 * b + lane;
         const bool on = 32 * b < chunk && i < numel;
-        e[b] = on ? __ldcg(topk_ids + i) : -1;  // (negative also: a row that holds nothing)
-        wt[b] = on ? __ldcg(topk_weights + i) : 0.0f;
+        e[b] = on ? (logits ? ids_s[i] : __ldcg(topk_ids + i)) : -1;  // (negative also: a row that holds nothing)
+        wt[b] = on ? (logits ? wts_s[i] : __ldcg(topk_weights + i)) : 0.0f;
     }
 #pragma unroll
     for (int b = 0; b < NB; ++b) {

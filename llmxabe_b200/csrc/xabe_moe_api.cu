@@ -981,7 +981,7 @@ int launch_route_and_dispatch(xabe_moe* m, cudaStream_t st, const float* logits)
         // decode widths: one single-CTA launch
         const size_t smem = dispatch_small_smem((int)g.num_experts);
         const float* fused_logits = logits;
-        if (logits && g.max_tokens > 8) {  // route on many SMs first
+        if (logits && g.max_tokens > (uint32_t)kDispatchRouted) {  // route on many SMs first
             CUDA_TRY(launch_pdl(overlap_of(m), k_route, dim3((g.max_tokens + 7) / 8), dim3(256), 0, st, logits,
                                 (const int*)m->valid_tokens, (int)g.num_experts, (int)g.experts_per_token,
                                 m->topk_ids, m->topk_weights));
