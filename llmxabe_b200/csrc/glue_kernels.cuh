@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(256 * PARTS, 1) k_router_logits_regw(const flo
     constexpr int kPairs = kRrStageTokens / kRrTokens;  // accumulator sets per ring stage
     const int part = threadIdx.x >> 8, tid = threadIdx.x & 255;
     float* group_tot = xs + kRrStages * kRrStageTokens * hidden + part * (2 * kPairs * kRrOutputs * 8);  // [2 stages][sets][32][8]
-    __shared__ __align__(8) uint64_t full[kRrStages];
+    __shared__ __align__(8) uint64_t full[kRrStages], wbar;
     const int e0 = (blockIdx.x * PARTS + part) * NE;
     const int live = *valid_tokens;
     // this CTA's tokens: a contiguous range, a whole number of stages except at the end of the batch
@@ -456,18 +456,27 @@ __global__ void __launch_bounds__(256 * PARTS, 1) k_router_logits_regw(const flo
                      &full[k % kRrStages]);
     };
     const int n_stages = stage1 - stage0;
+    // The CTA's expert rows come through the ring's memory first: a lane's slots hold the rows in an order of
+    // its own, which read directly would cost a sector per lane (23.4 instead of 16.8 us at 333 tokens).
     if (threadIdx.x == 0) {
         for (int i = 0; i < kRrStages; ++i) mbar_init(&full[i], 1);
+        mbar_init(&wbar, 1);
         fence_mbar_init();
-        for (int k = 0; k < min(kRrStages, n_stages); ++k) issue(k);
+        constexpr uint32_t bytes = (uint32_t)(NE * PARTS) * hidden * 4u;
+        mbar_expect_tx(&wbar, bytes);
+        tma_bulk_g2s(xs, w + (size_t)blockIdx.x * PARTS * NE * hidden, bytes, &wbar);
     }
+    __syncthreads();  // the barriers are initialised
+    if (!__syncthreads_and(mbar_wait_bounded(&wbar, 0u, status))) return;
     const int se = tid & (NE - 1), su = (tid & 31) / NE;  // this lane's slot swizzle (warp_trees32_swizzled)
     float wr[NE][NI];
 #pragma unroll
     for (int e = 0; e < NE; ++e)
 #pragma unroll
-        for (int i = 0; i < NI; ++i) wr[e][i] = __ldg(w + (size_t)(e0 + (e ^ se)) * hidden + i * 256 + tid);
-    __syncthreads();  // the barriers are initialised
+        for (int i = 0; i < NI; ++i) wr[e][i] = xs[(part * NE + (e ^ se)) * hidden + i * 256 + tid];
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 0; k < min(kRrStages, n_stages); ++k) issue(k);
     if (!__syncthreads_and(mbar_wait_bounded(&full[0], 0u, status))) return;
     for (int k = 0; k < n_stages; ++k) {
         const int slot = k % kRrStages;
