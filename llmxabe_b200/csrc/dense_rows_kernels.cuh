@@ -23,8 +23,11 @@
 // scale applied to the step's fp32 result, fp32 accumulation, spans in ascending order.  A token's
 // value depends only on its own activation row: the accumulator tiles of different groups never mix.
 //
-// Four loader warps fill the ring with 16-byte asynchronous copies (sixteen lanes per weight row);
-// every wait is bounded as in the other streaming kernels.
+// One thread fetches the weights as 2-D TMA boxes (R neighbouring rows make one row of the tensor map
+// where a row is not a multiple of 16 bytes, see pf_row_group; the rows of a box are then R apart), three warps
+// the activation rows with 16-byte asynchronous copies.  What bounds it is instruction issue: with the
+// weights copied sixteen bytes per lane by four warps those copies were 30 % of the instructions (a layer of
+// one token 69.9 -> 64.5 us, of 43 tokens 138 -> 133).  Every wait is bounded as in the other streaming kernels.
 #pragma once
 
 #include "prefill_kernels.cuh"
@@ -32,7 +35,7 @@
 
 namespace xabe {
 
-constexpr int kDrLoadWarps = 4;
+constexpr int kDrLoadWarps = 4;                                        // warp 0: weights, 1-3: activations
 constexpr int kDrConsumerWarps = kStreamConsumerWarps;                 // two groups of eight
 constexpr int kDrThreads = 32 * (kDrLoadWarps + kDrConsumerWarps);     // 640
 constexpr int kDrStageRows = 128;                                      // weight row-spans per stage
@@ -42,8 +45,8 @@ constexpr int kDrXPitch = 512 + 32;  // bytes between the activation rows of a s
 constexpr int kDrMaxTokens = 64;
 
 struct DenseRowsLaunch {
-    const uint8_t* w_a;  // gate (or down)
-    const uint8_t* w_b;  // up (MODE_GATEUP)
+    CUtensorMap tm_a;    // gate (or down) bytes
+    CUtensorMap tm_b;    // up (MODE_GATEUP)
     int rows, k;         // output rows per matrix, contraction length
     const int* valid_tokens;
     const __half* x;     // [tokens][k]
@@ -53,14 +56,18 @@ struct DenseRowsLaunch {
     int max_tokens;
     int n_stages;
     int x_rows;          // activation rows a stage holds (8 x groups)
-    int raw_pitch;       // bytes between the weight rows of a stage: 240 (Q6_K) or 304 (Q8_0), see dense_rows_pitch
+    int raw_pitch;       // bytes between the weight rows of a stage: the box width, 240 (Q6_K) or 272 (Q8_0)
+    int row_group;       // R: neighbouring rows per row of the tensor maps
     int k_splits;        // MODE_DOWN: shares of the contraction
 };
 
-// A row's span is copied as the 16-byte units that cover it (210 bytes starting up to 14 bytes into
-// a unit: 14 units; 272 bytes: 18), and the rows of a stage sit 240 / 304 bytes apart: 60 / 76
-// words, so the eight rows a fragment load touches start four banks apart and cover all 32 banks.
-__host__ __device__ inline int dense_rows_pitch(int quant) { return quant == QUANT_Q6K ? 240 : 304; }
+// 240 / 272 bytes are 60 / 68 words: the eight rows a fragment load touches start four banks apart and cover
+// all 32 banks.  A stage holds the R classes of its rows one after the other: slot c * (n / R) + i of n rows is
+// row i * R + c.
+__device__ __forceinline__ int dense_row_of_slot(int slot, int n, int R) {
+    const int per = n / R, c = slot / per;
+    return (slot - c * per) * R + c;
+}
 
 __host__ __device__ inline uint32_t dense_rows_stage_bytes(int raw_pitch, int x_rows) {
     return (uint32_t)(kDrStageRows * raw_pitch + x_rows * kDrXPitch);
@@ -183,20 +190,14 @@ __device__ __forceinline__ void dense_consume(const DenseRowsLaunch& L, uint8_t*
         int s0, s1;
         share(ks, s0, s1);
         const int first_row = rb * UNIT_ROWS + gi * (UNIT_ROWS / 2);
-        // fragment rows g and g + 8 of this warp: where they sit in a stage and in the matrices
-        int ra_slot, rb_slot;
-        uintptr_t ga, gb;  // global byte addresses of the two rows (only their low bits are used)
-        if (MODE == MODE_GATEUP) {
-            ra_slot = w * 8 + g;
-            rb_slot = 64 + w * 8 + g;
-            ga = (uintptr_t)(L.w_a + (size_t)(first_row + w * 8 + g) * row_bytes);
-            gb = (uintptr_t)(L.w_b + (size_t)(first_row + w * 8 + g) * row_bytes);
-        } else {
-            ra_slot = w * 16 + g;
-            rb_slot = w * 16 + g + 8;
-            ga = (uintptr_t)(L.w_a + (size_t)(first_row + ra_slot) * row_bytes);
-            gb = (uintptr_t)(L.w_a + (size_t)(first_row + rb_slot) * row_bytes);
-        }
+        // fragment rows g and g + 8 of this warp: where they sit in a stage and in the matrices (a warp's rows
+        // are of one class, so they share one alignment)
+        constexpr int kBlock = MODE == MODE_GATEUP ? 64 : 128;  // rows of one matrix per stage
+        const int ra_slot = MODE == MODE_GATEUP ? w * 8 + g : w * 16 + g;
+        const int rb_slot = MODE == MODE_GATEUP ? 64 + w * 8 + g : w * 16 + g + 8;
+        const int R = L.row_group, x0 = ra_slot / (kBlock / R) * (int)row_bytes;
+        const int row_a = first_row + dense_row_of_slot(ra_slot, kBlock, R);
+        const int row_b = MODE == MODE_GATEUP ? row_a : first_row + dense_row_of_slot(rb_slot, kBlock, R);
         float acc[NG][4];
 #pragma unroll
         for (int q = 0; q < NG; ++q)
@@ -205,8 +206,10 @@ __device__ __forceinline__ void dense_consume(const DenseRowsLaunch& L, uint8_t*
         for (int s = s0; s < s1; ++s) {
             if (!stream_wait(&full[st], use & 1, abortp, L.status)) return;
             const uint8_t* slot = smem + (uint32_t)st * stage_bytes;
-            const uint8_t* pa = slot + (uint32_t)ra_slot * L.raw_pitch + (uint32_t)((ga + (size_t)s * span_b) & 15u);
-            const uint8_t* pb = slot + (uint32_t)rb_slot * L.raw_pitch + (uint32_t)((gb + (size_t)s * span_b) & 15u);
+            const int x = x0 + s * span_b;
+            const uint8_t* pa = slot + (uint32_t)ra_slot * L.raw_pitch +
+                                (uint32_t)(x - rows_box_start(x, R * (int)row_bytes, L.raw_pitch));
+            const uint8_t* pb = pa + (uint32_t)(rb_slot - ra_slot) * L.raw_pitch;
             const uint8_t* xs = slot + (uint32_t)(kDrStageRows * L.raw_pitch) + (uint32_t)g * kDrXPitch;
             // every row pitch is a multiple of four bytes (checked by the host), so the two rows and
             // all lanes of the warp share one word alignment
@@ -227,7 +230,7 @@ __device__ __forceinline__ void dense_consume(const DenseRowsLaunch& L, uint8_t*
         }
         if (MODE == MODE_GATEUP) {
             // SwiGLU of this warp's eight rows: acc[.][0..1] gate, acc[.][2..3] up, columns 2t and 2t + 1
-            const int row = first_row + w * 8 + g;
+            const int row = row_a;
 #pragma unroll
             for (int q = 0; q < NG; ++q)
 #pragma unroll
@@ -239,7 +242,7 @@ __device__ __forceinline__ void dense_consume(const DenseRowsLaunch& L, uint8_t*
                     }
                 }
         } else {
-            const int row_lo = first_row + ra_slot, row_hi = first_row + rb_slot;
+            const int row_lo = row_a, row_hi = row_b;
             float* dst = L.out + (size_t)ks * L.max_tokens * L.rows;
 #pragma unroll
             for (int q = 0; q < NG; ++q)
@@ -255,9 +258,9 @@ __device__ __forceinline__ void dense_consume(const DenseRowsLaunch& L, uint8_t*
     }
 }
 
-// grid: number of SMs; block: kDrThreads (warps 0-1 load, warps 2-17 consume).
+// grid: number of SMs; block: kDrThreads (warps 0-3 load, warps 4-19 consume).
 template <int MODE, int QUANT, int NG>
-__global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L) {
+__global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(const __grid_constant__ DenseRowsLaunch L) {
     pdl_launch_dependents();
     extern __shared__ __align__(128) uint8_t dr_raw[];
     __shared__ int abort_flag;
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int i = 0; i < S; ++i) {
-            mbar_init(&full[i], kDrLoadWarps * 32);  // every loader lane's copies of the stage have landed
+            mbar_init(&full[i], 1 + (kDrLoadWarps - 1) * 32);  // the weight boxes, and every other loader lane's copies
             mbar_init(&empty[i], kStreamGroupWarps);
         }
         fence_mbar_init();
@@ -293,11 +296,16 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
 
     if (warp < kDrLoadWarps) {
         // -------------------------------- loaders --------------------------------
-        const int LL = warp * 32 + lane;                                  // 0 .. 127
-        constexpr int ROWS_PER_PASS = kDrLoadWarps * 2;                   // sixteen lanes per weight row
-        const int wrow = LL >> 4, wpart = LL & 15;
-        const int xrow = LL >> 5, xpart = LL & 31;                        // activations: thirty-two lanes per row
-        int st = 0, valid = -1;
+        const bool weights = warp == 0;
+        if (weights && lane != 0) return;
+        int valid = 0;
+        if (!weights) {  // the weights are constant; the activations have a producer
+            pdl_wait();
+            valid = min(*L.valid_tokens, L.max_tokens);
+        }
+        constexpr int HALVES = MODE == MODE_GATEUP ? 2 : 1, ROWS_EACH = kDrStageRows / HALVES;
+        const int R = L.row_group, per = ROWS_EACH / R;
+        int st = 0;
         uint32_t use = 0;
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
             const int rb = u / KS, ks = u - rb * KS;
@@ -311,43 +319,22 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
                         return;
                     }
                     uint8_t* slot = smem + (uint32_t)st * stage_bytes;
-                    const uint32_t slot32 = smem_u32(slot);
-                    const int first_row = rb * UNIT_ROWS + gi * (UNIT_ROWS / 2);
-                    // this lane's rows of the stage: wrow, wrow + 8, ...; the source pointer and the
-                    // destination advance by a constant per pass
-                    constexpr int HALVES = MODE == MODE_GATEUP ? 2 : 1;
-                    constexpr int ROWS_EACH = kDrStageRows / HALVES;
-#pragma unroll
-                    for (int hm = 0; hm < HALVES; ++hm) {
-                        const uint8_t* src = (hm == 0 ? L.w_a : L.w_b) + (size_t)(first_row + wrow) * row_bytes +
-                                             (size_t)s * span_b;
-                        uint32_t dst = slot32 + (uint32_t)(hm * ROWS_EACH + wrow) * L.raw_pitch + (uint32_t)wpart * 16u;
-                        const size_t src_step = (size_t)ROWS_PER_PASS * row_bytes;
-                        const uint32_t dst_step = (uint32_t)ROWS_PER_PASS * L.raw_pitch;
-#pragma unroll 4
-                        for (int r = 0; r < ROWS_EACH / ROWS_PER_PASS; ++r) {
-                            const uint32_t off = (uint32_t)((uintptr_t)src & 15u);
-                            const uint32_t chunks = (off + (uint32_t)span_b + 15u) >> 4;  // never past the span's last unit
-                            const uint8_t* win = src - off + wpart * 16;
-                            if ((uint32_t)wpart < chunks) cp_async16(dst, win, 16u);
-                            if (QUANT != QUANT_Q6K && (uint32_t)wpart + 16u < chunks) cp_async16(dst + 256u, win + 256, 16u);
-                            src += src_step;
-                            dst += dst_step;
+                    if (weights) {
+                        const int y = (rb * UNIT_ROWS + gi * (UNIT_ROWS / 2)) / R;
+                        mbar_expect_tx(&full[st], (uint32_t)(kDrStageRows * L.raw_pitch));
+#pragma unroll 1
+                        for (int c = 0; c < R; ++c, slot += per * L.raw_pitch) {
+                            const int x = rows_box_start(c * (int)row_bytes + s * span_b, R * (int)row_bytes, L.raw_pitch) >> 2;
+                            tma_load_box_2d(slot, &L.tm_a, x, y, &full[st]);
+                            if (MODE == MODE_GATEUP) tma_load_box_2d(slot + ROWS_EACH * L.raw_pitch, &L.tm_b, x, y, &full[st]);
                         }
+                    } else {
+                        const uint32_t x32 = smem_u32(slot) + (uint32_t)(kDrStageRows * L.raw_pitch);
+                        for (int tk = warp - 1; tk < valid; tk += kDrLoadWarps - 1)  // thirty-two lanes per row
+                            cp_async16(x32 + (uint32_t)tk * kDrXPitch + (uint32_t)lane * 16u,
+                                       L.x + (size_t)tk * L.k + (size_t)s * kSpanElems + lane * 8, 16u);
+                        cp_async_arrive_noinc(&full[st]);
                     }
-                    if (valid < 0) {  // the first stage's weights are on their way; the activations have a producer
-                        pdl_wait();
-                        valid = min(*L.valid_tokens, L.max_tokens);
-                        if (valid <= 0) {
-                            asm volatile("cp.async.wait_all;" ::: "memory");
-                            return;
-                        }
-                    }
-                    const uint32_t x32 = slot32 + (uint32_t)(kDrStageRows * L.raw_pitch);
-                    for (int tk = xrow; tk < valid; tk += kDrLoadWarps)
-                        cp_async16(x32 + (uint32_t)tk * kDrXPitch + (uint32_t)xpart * 16u,
-                                   L.x + (size_t)tk * L.k + (size_t)s * kSpanElems + xpart * 8, 16u);
-                    cp_async_arrive_noinc(&full[st]);
                     if (++st == S) {
                         st = 0;
                         ++use;
@@ -361,8 +348,7 @@ __global__ void __launch_bounds__(kDrThreads, 1) k_dense_rows(DenseRowsLaunch L)
 
     // ---------------------------------- consumers ----------------------------------
     pdl_wait();
-    const int valid = min(*L.valid_tokens, L.max_tokens);
-    if (valid <= 0) return;
+    const int valid = min(*L.valid_tokens, L.max_tokens);  // (none: nothing is stored)
     // As many groups as hold live tokens: a handle of 64 with 43 live ones runs the code for six groups, not for
     // eight (164 -> 149 us per layer).  The code is chosen once per launch; a bound inside the loops cost more
     // than it saved.

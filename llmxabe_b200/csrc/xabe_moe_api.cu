@@ -660,8 +660,9 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
             P.status = m->status;
             P.max_tokens = (int)g.max_tokens;
             P.x_rows = 8 * ng;
-            auto shape = [&](int quant) {
-                P.raw_pitch = dense_rows_pitch(quant == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
+            auto shape = [&](int quant, size_t row_bytes) {
+                P.raw_pitch = (int)rows_box_bytes(quant == XABE_QUANT_Q6_K ? QUANT_Q6K : QUANT_Q8_0);
+                P.row_group = pf_row_group((uint32_t)row_bytes);
                 P.n_stages = 2;
                 for (int S = kDrMaxStages; S >= 2; --S)
                     if (dense_rows_smem(S, P.raw_pitch, P.x_rows) <= 200u * 1024u) {
@@ -670,26 +671,29 @@ int run_experts(xabe_moe* m, cudaStream_t st, const MlpWeights& routed, const Ml
                     }
                 return dense_rows_smem(P.n_stages, P.raw_pitch, P.x_rows);
             };
-            P.w_a = (const uint8_t*)shared.gate.dev_bytes;
-            P.w_b = (const uint8_t*)shared.up.dev_bytes;
+            auto map = [&](CUtensorMap* tm, const xabe_quant_tensor& t, uint64_t rows, size_t row_bytes, uint32_t block) {
+                return make_bytes_map(tm, t.dev_bytes, rows / P.row_group, row_bytes * P.row_group, (uint32_t)P.raw_pitch,
+                                      block / (uint32_t)P.row_group);
+            };
+            uint32_t smem = shape(qs, rb_gu);
+            int rc = map(&P.tm_a, shared.gate, g.intermediate, rb_gu, kDrStageRows / 2);
+            if (!rc) rc = map(&P.tm_b, shared.up, g.intermediate, rb_gu, kDrStageRows / 2);
+            if (rc) return rc;
             P.rows = (int)g.intermediate;
             P.k = (int)g.hidden;
             P.x = m->normed_h;
             P.inter = m->inter_shared;
             P.k_splits = 1;
-            uint32_t smem = shape(qs);
-            int rc = launch_dense_rows<MODE_GATEUP>(m, st, P, qs, ng, smem);
-            if (rc) return rc;
+            if ((rc = launch_dense_rows<MODE_GATEUP>(m, st, P, qs, ng, smem))) return rc;
             if (mark_between >= 0) prof_mark(m, st, mark_between);
-            P.w_a = (const uint8_t*)shared.down.dev_bytes;
-            P.w_b = nullptr;
             P.rows = (int)g.hidden;
             P.k = (int)g.intermediate;
             P.x = m->inter_shared;
             P.inter = nullptr;
             P.k_splits = m->dense_k_splits;
             P.out = P.k_splits > 1 ? m->dense_partial : shexp_out;
-            smem = shape(qd);
+            smem = shape(qd, rb_dn);
+            if ((rc = map(&P.tm_a, shared.down, g.hidden, rb_dn, kDrStageRows))) return rc;
             if ((rc = launch_dense_rows<MODE_DOWN>(m, st, P, qd, ng, smem))) return rc;
             if (P.k_splits > 1) {
                 CUDA_TRY(launch_pdl(overlap_of(m), k_sum_k_splits, dim3(g.max_tokens, (g.hidden + 255) / 256),
