@@ -109,6 +109,9 @@ cudaError_t launch_pdl(Overlap overlap, void (*kern)(KArgs...), dim3 grid, dim3 
 // Wide passes only take the tcgen05 prefill kernels; the launch shape comes from max_tokens.
 constexpr uint32_t kPrefillMinTokens = 512;
 
+// Handles from this width up (and below kPrefillMinTokens) have a stream for the shared expert (see forks_shared).
+constexpr uint32_t kForkMinTokens = 16;
+
 // Handles narrower than this fold the block's last stage into the down projection's launch.
 constexpr uint32_t kTailMaxTokens = 16;
 
@@ -574,7 +577,7 @@ struct DenseTail {
 // -> 1476 us), so handles under 16 tokens keep the mixed launch.
 bool forks_shared(const xabe_moe* m, const xabe_moe_layer_weights* w) {
     const auto& g = m->g;
-    return m->side && g.max_tokens >= 16 && !m->prof_on && !m->pdl && !m->force_tile_kernels &&
+    return m->side && !m->prof_on && !m->pdl && !m->force_tile_kernels &&
            (w->gate_exps.quant != w->shared_gate.quant || w->down_exps.quant != w->shared_down.quant) &&
            !prefill_applies(m, (int)g.intermediate, (int)g.hidden, (int)g.hidden, (int)g.intermediate);
 }
@@ -1235,7 +1238,7 @@ int xabe_moe_create(const xabe_moe_geometry* geometry, int device, int scope, fl
         A(dev_alloc(&m->routed, T * H));
         A(dev_alloc(&m->gate, T));
     }
-    if (scope == XABE_SCOPE_ROUTED) {
+    if (scope == XABE_SCOPE_ROUTED && g.max_tokens >= kForkMinTokens && g.max_tokens < kPrefillMinTokens) {
         A(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
         A(cudaEventCreateWithFlags(&m->ev_fork, cudaEventDisableTiming));
         A(cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming));

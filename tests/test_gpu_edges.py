@@ -1,0 +1,134 @@
+"""The kernels' edges: sizes at which a tile, a ring stage, a token group or a cluster's share ends.
+
+Bounds: whole numbers and rows that the contract calls bit-identical are compared exactly; outputs of the
+tcgen05 kernels against the oracle within rel-L2 1e-3 (f16 activations and intermediates 2e-4 each, f16
+weights 2e-4: root sum of squares 3.5e-4, times a margin of about three), as everywhere in these tests.
+"""
+import numpy as np
+import pytest
+
+from helpers import bits, device_layer, oracle_layer, run_block
+
+pytestmark = pytest.mark.gpu
+REL_L2 = 1e-3
+
+
+@pytest.mark.parametrize("vocab", [1, 7, 8, 9, 511, 4097, 32769])
+def test_argmax_over_a_cluster_at_the_ends_of_its_shares(oracle, vocab):
+    import torch
+    from llmxabe_b200.lm_head import LmHeadGeometry, LmHeadKernels
+    T = 5
+    k = LmHeadKernels(LmHeadGeometry(256, vocab, T))
+    v = np.random.default_rng(vocab).standard_normal((T, vocab)).astype(np.float32)
+    share = -(-vocab // 8)
+    v[1, min(vocab - 1, share)] = v[1, vocab - 1] = 9.0          # a tie between two CTAs' shares
+    v[2, max(0, min(vocab, share) - 1)] = 9.0                    # the last element of the first share
+    v[3] = -1.0                                                  # all equal
+    v[4, vocab - 1] = 9.0
+    out = torch.zeros(T, dtype=torch.int32, device="cuda")
+    k.argmax(torch.from_numpy(v).cuda(), T, out)
+    assert out.cpu().tolist() == [oracle.argmax(v[t]) for t in range(T)]
+
+
+@pytest.mark.parametrize("hidden,inter", [(512, 256), (1024, 512), (2048, 512)])
+@pytest.mark.parametrize("quants", [(0, 0), (1, 1), (0, 1)])
+def test_prefill_tiles_at_their_edges(oracle, hidden, inter, quants):
+    """Rows of 210, 420, 840 and 1680 bytes (8, 4, 2 and 1 of them per row of a tensor map) and of whole 16-byte
+    units; expert tiles of every remainder around 16, 32, 64 and 128 tokens."""
+    from llmxabe_b200 import synth
+    from llmxabe_b200.moe import MoeBlock, MoeGeometry
+    T = 260
+    L = synth.moe_layer(seed=70, num_experts=4, top_k=2, hidden=hidden, inter=inter, routed_quant=quants[0],
+                        shared_quant=quants[1], zipf=True)
+    x = synth.activations(T, hidden, seed=70)
+    w = device_layer(L)
+    want = oracle.moe_block_forward(oracle_layer(oracle, L), x, dev_order=True)
+    blk = MoeBlock(MoeGeometry(4, 2, hidden, inter, 16, T))
+    blk.moe.force_prefill_path(True)
+    for tokens in (1, 15, 16, 17, 33, 63, 64, 65, 127, 128, 129, 257, 260):
+        got = run_block(blk, w, x[:tokens], T)
+        assert blk.moe.device_status() == 0 and got["untouched"]
+        for name in ("routed", "shexp", "l_out"):
+            r = oracle.compare(got[name], want[name][:tokens])
+            assert r.non_finite_count == 0 and r.rel_l2 <= REL_L2, f"{tokens} {name}: {r}"
+
+
+def test_dense_rows_do_not_depend_on_the_live_groups():
+    """One handle of 64: a row's value is the same whichever number of eight-token groups is live."""
+    import torch
+    from llmxabe_b200 import synth
+    from llmxabe_b200.moe import DenseFfnBlock, MoeGeometry, QuantTensor
+    width = 64
+    for hidden, inter in ((2560, 2048), (5120, 1024)):
+        post_norm, gate, up, down = synth.dense_layer(seed=71, hidden=hidden, inter=inter, quant=0)
+        qt = [QuantTensor(torch.from_numpy(a).cuda(), 0) for a in (gate, up, down)]
+        blk = DenseFfnBlock(MoeGeometry(1, 1, hidden, inter, 64, width))
+        res = torch.from_numpy(synth.activations(width, hidden, seed=71)).cuda()
+        pn = torch.from_numpy(post_norm).cuda()
+
+        def run(tokens):
+            ffn, lo = (torch.full((width, hidden), 5.0, device="cuda") for _ in range(2))
+            blk.forward(pn, *qt, res, tokens, ffn, lo)
+            assert blk.moe.device_status() == 0
+            assert bool((lo[tokens:] == 5.0).all().item())
+            return lo[:tokens].cpu().numpy()
+
+        full = run(width)
+        for tokens in (0, 1, 8, 9, 16, 17, 25, 33, 41, 49, 56, 57):
+            assert (bits(run(tokens)) == bits(full[:tokens])).all(), (hidden, inter, tokens)
+
+
+@pytest.mark.parametrize("experts,tokens", [(3, 1), (3, 40), (256, 31), (256, 33), (512, 64), (512, 255), (512, 256)])
+def test_one_pass_dispatch_with_crowded_experts(oracle, experts, tokens):
+    """The one-CTA dispatch from 1 to 2048 pairs, most of them on one expert, its groups of eight included."""
+    import torch
+    from llmxabe_b200.moe import MoeGeometry, MoeKernels
+    K = 3 if experts == 3 else 8
+    g = MoeGeometry(experts, K, 256, 256, 16, tokens)
+    k = MoeKernels(g)
+    rng = np.random.default_rng(experts + tokens)
+    ids = np.empty((tokens, K), np.int32)
+    for t in range(tokens):
+        other = rng.choice(np.arange(1, experts), K - 1, replace=False)
+        ids[t] = rng.permutation(np.concatenate(([0], other)))   # every token picks expert 0
+    k.set_valid_tokens(tokens)
+    k.build_dispatch(torch.from_numpy(ids).cuda(), torch.full((tokens, K), 1.0 / K, device="cuda"))
+    torch.cuda.synchronize()
+    b = k.buffers()
+    want = oracle.moe_align_block_size(ids, g.block_size, experts)
+    n = want.num_tokens_post_pad
+    assert int(b.num_tokens_post_pad.cpu().item()) == n
+    assert (b.sorted_token_ids.cpu().numpy()[:n] == want.sorted_token_ids).all()
+    assert (b.sorted_token_ids.cpu().numpy()[n:] == tokens * K).all()
+    assert (b.expert_ids.cpu().numpy()[: n // g.block_size] == want.expert_ids).all()
+
+
+@pytest.mark.parametrize("tokens,width", [(16, 16), (21, 64), (300, 300)])
+def test_shared_expert_beside_the_dispatch(oracle, tokens, width):
+    """Q6_K routed experts with a Q8_0 shared expert: the shared projections run on a stream of the handle's own,
+    eagerly and inside a replayed graph."""
+    import torch
+    from llmxabe_b200 import synth
+    from llmxabe_b200.moe import MoeBlock, MoeGeometry
+    L = synth.moe_layer(seed=72, num_experts=16, top_k=4, hidden=1024, inter=512, shared_quant=1, zipf=True)
+    x = synth.activations(tokens, 1024, seed=72)
+    w = device_layer(L)
+    blk = MoeBlock(MoeGeometry(16, 4, 1024, 512, 16, width))
+    got = run_block(blk, w, x, width)
+    assert blk.moe.device_status() == 0 and got["untouched"]
+    want = oracle.moe_block_forward(oracle_layer(oracle, L), x, dev_order=True)
+    for name in ("routed", "shexp", "l_out"):
+        r = oracle.compare(got[name], want[name])
+        assert r.non_finite_count == 0 and r.rel_l2 <= REL_L2, f"{name}: {r}"
+    res = torch.zeros(width, 1024, device="cuda")
+    res[:tokens] = torch.from_numpy(x).cuda()
+    ffn, lo = torch.zeros_like(res), torch.zeros_like(res)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        blk.forward(w, res, tokens, ffn, lo)
+    for _ in range(3):
+        lo.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert (bits(lo[:tokens].cpu().numpy()) == bits(got["l_out"])).all()
