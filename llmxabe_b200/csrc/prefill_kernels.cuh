@@ -13,8 +13,8 @@
 //   * sixteen unpack warps: a THREAD is a weight row.  It reads its row with
 //     16-byte shared loads (a 240- or 272-byte pitch is an odd number of 16-byte
 //     units: no bank conflicts), unpacks, scales, and writes f16 weights with
-//     tcgen05.st into a ring of four A stages in tensor memory (128 rows x 128
-//     contraction elements each).  One scale serves the sixteen weights of a
+//     tcgen05.st into a ring of four stages in tensor memory (64 contraction
+//     elements of both row tiles each; a span is one turn of the ring).  One scale serves the sixteen weights of a
 //     store, and the weights never pass through shared memory;
 //   * two warps bring the token rows of the tile (B operand) into 128-byte-swizzled
 //     shared-memory tiles: rows that lie one after the other (the down projection's
@@ -23,21 +23,23 @@
 //     measured: 97 clocks per four rows, 1.6 times the whole launch's time);
 //   * one thread issues tcgen05.mma (A from tensor memory, M128 K16, N = the
 //     tile's token count rounded up to 16);
-//   * four epilogue warps read finished accumulators (a thread = a weight row,
-//     so gate and up of an output meet in one thread), apply SwiGLU or the
-//     routing weight, and turn sixteen tokens at a time around in shared memory,
-//     so that a token's 128 outputs leave as one contiguous piece.
+//   * two teams of four epilogue warps read finished accumulators (a thread = a
+//     weight row, so gate and up of an output meet in one thread), apply SwiGLU or
+//     the routing weight, and turn sixteen tokens at a time around in shared
+//     memory, so that a token's 128 outputs leave as one contiguous piece.
 // Tiles of up to 64 tokens use half of the accumulator columns, so that the
 // epilogue of one tile runs under the next one's products.
 //
-// What bounds it: with few tokens per expert the unpack, 2.9 thread
-// instructions per weight (99 of them per 32 weights: 2.25 per pair of codes to
-// assemble and place, 1.5 to convert and scale, the rest loads and stores);
-// with 128 tokens per tile shared-memory bandwidth, of which the products take
-// 32 KB per 64 contraction elements (the B tile, once per row tile), the B fill
-// 16 KB, the raw bytes 16 KB in and 20 KB out.  The kernel this one replaced
-// kept both operands in shared memory: 16 KB of weight stores and 32 KB of
-// operand reads more per 64 elements of the same 256 rows.
+// What bounds it: nothing alone.  With 128 tokens per tile the products of a span
+// take 2048 clocks, its shared-memory traffic about 2600 (products 128 KB, token
+// rows 64 KB, raw bytes 61 KB in and 82 KB out, at 128 bytes a clock) and the unpack
+// 1600 issue slots per scheduler; a span takes 4200.  Leaving out one of the four
+// saves 5 to 20 % each, and the bare pipeline of barriers takes 40 to 60 % of the
+// time.  Measured against the kernel with both operands in shared memory it replaced
+// (gate/up + down launches): 16384 tokens, top-8 1612 -> 1240 us, 2048 tokens 417 -> 317,
+// dense block at 4096 tokens 2523 -> 2340 (where the power limit of a long run takes
+// most of it back).  Tiles of 64 tokens for the short contraction of the routed down
+// projection, whose epilogue would then run under the next tile: 549 -> 667 us.
 //
 // Numerics: weights are rounded to f16 after the fp32-exact code is multiplied
 // by the f16-rounded group scale (times 256, undone in the epilogue, which
