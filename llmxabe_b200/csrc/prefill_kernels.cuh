@@ -37,8 +37,7 @@
 // saves 5 to 20 % each, and the bare pipeline of barriers takes 40 to 60 % of the
 // time.  Measured against the kernel with both operands in shared memory it replaced
 // (gate/up + down launches): 16384 tokens, top-8 1612 -> 1240 us, 2048 tokens 417 -> 317,
-// dense block at 4096 tokens 2523 -> 2340 (where the power limit of a long run takes
-// most of it back).  Tiles of 64 tokens for the short contraction of the routed down
+// dense block at 4096 tokens 2867 -> 2604 a layer.  Tiles of 64 tokens for the short contraction of the routed down
 // projection, whose epilogue would then run under the next tile: 549 -> 667 us.
 //
 // Numerics: weights are rounded to f16 after the fp32-exact code is multiplied
@@ -297,8 +296,13 @@ __device__ __forceinline__ PfTile pf_tile(const PrefillLaunch& L, int t, int n_r
         T.first = __ldg(it + 1);
         T.ncols = __ldg(it + 2);
     } else {
+        // The shared expert's (or the dense block's) token tiles are the faster index: the CTAs at work then share
+        // few weight rows, which L2 keeps, instead of walking all of them once per token tile (the dense gate/up
+        // matrices, 146 MB, came from HBM 32 times at 4096 tokens: 2861 -> 2604 us a layer, most of it power).
+        const int s = t - n_routed * L.row_units, n_shared = (valid + kPfTileN - 1) / kPfTileN;
+        T.bx = s / n_shared;
         T.expert = 0;
-        T.first = (y - n_routed) * kPfTileN;
+        T.first = (s - T.bx * n_shared) * kPfTileN;
         T.ncols = min(kPfTileN, valid - T.first);
     }
     return T;
